@@ -239,9 +239,12 @@ int read_scalars(pal_handle* h) {
   return PAL_OK;
 }
 
-// om / fnm1 from the natural columns into om_p / fm_p (to_perm) or back.
-int om_layout(pal_handle* h, bool to_perm) {
+// om / fnm1 from the natural columns into om_p / fm_p (to_perm) or back.  An
+// LS-IMEX-RK3 step's first stage does not read fnm1 (its weight is 0) and its
+// last writes all of it, so only om goes in.
+int om_layout(pal_handle* h, bool to_perm, int method) {
   StepArgs a = base_args(h);
+  if (to_perm && method == PAL_LS_IMEX_RK3) a.flags = pal::F_NO_FM_IN;
   if (to_perm)
     h->ck->to_perm(a, h->stream);
   else
@@ -692,9 +695,9 @@ int pal_step_rk3(pal_handle* h) {
   if (int rc = resolve_velocity(h)) return rc;
   if (h->state != ST_U) return fail(h, PAL_ERR_STATE, "LS-IMEX-RK3 step needs the physical velocity");
   // three column passes: worth the butterfly-major order and its two conversions
-  if (int rc = om_layout(h, true)) return rc;
+  if (int rc = om_layout(h, true, PAL_LS_IMEX_RK3)) return rc;
   const int rc = one_step(h, PAL_LS_IMEX_RK3, false, false, true);
-  const int rc2 = om_layout(h, false);
+  const int rc2 = om_layout(h, false, PAL_LS_IMEX_RK3);
   return rc != PAL_OK ? rc : rc2;
 }
 
@@ -725,10 +728,10 @@ int pal_step(pal_handle* h, int method, int nsteps, int update, int final_update
     // conversions (~60 us each at N=4096) cost less than one step's three
     // natural-order column passes (~370 us more).
     auto record = [&]() -> int {
-      if (int rc = om_layout(h, true)) return rc;
+      if (int rc = om_layout(h, true, method)) return rc;
       int rc = PAL_OK;
       for (int j = 0; j < nsteps && rc == PAL_OK; ++j) rc = one_step(h, method, upd[j] != 0, true, true);
-      const int rc2 = om_layout(h, false);
+      const int rc2 = om_layout(h, false, method);
       return rc != PAL_OK ? rc : rc2;
     };
     const char* env = std::getenv("PAL_STEP_GRAPHS");
@@ -1105,7 +1108,7 @@ int pal_profile_kernels(pal_handle* h, int method, int nsteps, double* ms_row, d
     }
   }
   int k = 0;
-  if (rc == PAL_OK) rc = om_layout(h, true);  // the pass as pal_step runs it
+  if (rc == PAL_OK) rc = om_layout(h, true, method);  // the pass as pal_step runs it
   if (rc == PAL_OK) {
     cudaEventRecord(ev[k++], h->stream);
     for (int j = 0; j < nsteps && rc == PAL_OK; ++j) {
@@ -1119,7 +1122,7 @@ int pal_profile_kernels(pal_handle* h, int method, int nsteps, double* ms_row, d
       }
       if (rc == PAL_OK) h->it += 1;
     }
-    const int rc2 = om_layout(h, false);
+    const int rc2 = om_layout(h, false, method);
     if (rc == PAL_OK) rc = rc2;
   }
   double tr = 0.0, tc = 0.0;

@@ -46,11 +46,11 @@ struct FusedSize {
   }
   template <int NT, bool TO>
   static __device__ __forceinline__ void perm(const StepArgs& a, Blk bk) {
-    om_perm_body<float, PLC, TO, NT>(a, bk);
+    om_perm_body<float, PLC, TO, NT>(a, bk, true, (a.flags & F_NO_FM_IN) == 0);
   }
   static constexpr size_t smem_row = size_t(PLR::PADM) * VR * sizeof(float2);
   static constexpr size_t smem_col = size_t(PLC::PADM) * 2 * sizeof(float2);
-  static constexpr size_t smem_perm = size_t(2) * (2 * PLC::M / 3) * sizeof(float2);
+  static constexpr size_t smem_perm = PermTile<float, PLC>::smem;
 };
 
 // The group of block b and the block's position in it.

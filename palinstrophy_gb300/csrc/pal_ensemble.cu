@@ -149,18 +149,23 @@ int fused_args(const pal_ensemble* e, pal::FusedArgs& f, PerMember per_member, A
   return blocks;
 }
 
-int om_layout(pal_ensemble* e, bool to_perm) {
+// Only om goes in for LS-IMEX-RK3, whose first stage does not read fnm1.
+int om_layout(pal_ensemble* e, bool to_perm, int method) {
+  auto args = [&](const Group& g) {
+    StepArgs a = group_args(e, g);
+    if (to_perm && method == PAL_LS_IMEX_RK3) a.flags = pal::F_NO_FM_IN;
+    return a;
+  };
   if (e->fused) {
     pal::FusedArgs f;
-    const int nb = fused_args(e, f, [](const Group& g) { return g.Nh; },
-                              [&](const Group& g) { return group_args(e, g); });
+    const int nb = fused_args(e, f, [](const Group& g) { return g.Nh; }, args);
     (to_perm ? e->fused->to_perm : e->fused->from_perm)(f, nb, e->stream);
     cudaError_t c = cudaGetLastError();
     if (c != cudaSuccess) return efail(e, PAL_ERR_CUDA, std::string("ensemble om order: ") + cudaGetErrorString(c));
     return PAL_OK;
   }
   for (Group& g : e->groups) {
-    StepArgs a = group_args(e, g);
+    StepArgs a = args(g);
     if (to_perm)
       g.ck->to_perm(a, e->stream);
     else
@@ -568,10 +573,10 @@ int pal_ensemble_step(pal_ensemble* e, int method, int nsteps, int update, int u
   upd[nsteps] = pending;
   for (bool b : upd) key += b ? '1' : '0';
   auto record = [&]() -> int {
-    if (int rc = om_layout(e, true)) return rc;
+    if (int rc = om_layout(e, true, method)) return rc;
     for (int j = 0; j < nsteps; ++j)
       if (int rc = launch_step(e, method, upd[j])) return rc;
-    if (int rc = om_layout(e, false)) return rc;
+    if (int rc = om_layout(e, false, method)) return rc;
     if (upd[nsteps])
       if (int rc = launch_stats(e, pal::F_UPDATE_DT)) return rc;
     return PAL_OK;

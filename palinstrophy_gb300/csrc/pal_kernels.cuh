@@ -1595,54 +1595,78 @@ __global__ void __launch_bounds__(NT, MINB) k_col_tma(StepArgs a0, const __grid_
 
 // om / fnm1 between the natural [kx][z] columns and the butterfly-major
 // columns of the column plan PL (om_p, fm_p; only the N in-band entries of each
-// M-element column are written or read).  One block per kx column; the column
-// passes through shared memory, so both the natural and the butterfly-major
-// side are read and written in consecutive order.
+// M-element column are written or read).  A block moves one array's column kx
+// through shared memory (both arrays in turn when `both`), so both the natural
+// and the butterfly-major side are read and written in consecutive order.
+//
+// HBM bounds it (read + write of each array).  Consecutive butterflies differ
+// in the digit next to the last, so their natural positions are PermTile::STEP
+// apart: without the pad slot after every STEP entries a warp's shared-memory
+// accesses all fell into one bank.  One array per block (grid.z) halves the
+// tile, so three to six blocks share an SM where one or two did.  F_NO_FM_IN:
+// fnm1 is left out (the first RK3 stage does not read it).  N=8192 FP32: 1030 /
+// 880 us before (to / from the butterfly-major order, both arrays), now 174 us
+// for om alone / 345 us (3.1 TB/s); N=4096 143 / 99 us before, now 32 / 56 us.
+template <typename T, class PL>
+struct PermTile {
+  static constexpr int N = 2 * PL::M / 3;
+  static constexpr int STEP = PL::NP >= 3 ? PL::weight(PL::NP - 2) : N;  // natural distance of butterflies b, b + 1
+  static constexpr int SLOTS = N + (STEP < N ? N / STEP : 0);
+  static constexpr size_t smem = size_t(SLOTS) * sizeof(cplx<T>);
+  static __device__ __forceinline__ int slot(int z) { return STEP < N ? z + z / STEP : z; }
+};
 template <typename T, class PL, bool TO_PERM, int NT>
-__device__ __forceinline__ void om_perm_body(const StepArgs& a0, const Blk bk) {
+__device__ __forceinline__ void om_perm_column(cplx<T>* sm, cplx<T>* __restrict__ nat, cplx<T>* __restrict__ perm,
+                                               int tid) {
   using C = cplx<T>;
-  const StepArgs a = member_args(a0, sizeof(C), bk.y);
+  using PT = PermTile<T, PL>;
   constexpr int M = PL::M, N = 2 * M / 3, Nh = M / 3;
   constexpr int RP = PL::RP, FSTEP = PL::FSTEP;
-  extern __shared__ __align__(128) unsigned char smraw[];
-  C* so = reinterpret_cast<C*>(smraw);
-  C* sf = so + N;
-  const int kx = bk.x;
-  C* __restrict__ no = static_cast<C*>(a.om) + (size_t)kx * N;
-  C* __restrict__ nf = static_cast<C*>(a.fnm1) + (size_t)kx * N;
-  C* __restrict__ po = static_cast<C*>(a.om_p) + (size_t)kx * M;
-  C* __restrict__ pf = static_cast<C*>(a.fm_p) + (size_t)kx * M;
+  constexpr bool BAND_CT = (RP % 3 == 0) && ((RP / 3) % 2 == 0);  // the pad is the middle third of the j
   if constexpr (TO_PERM) {
-    for (int z = threadIdx.x; z < N; z += NT) {
-      so[z] = no[z];
-      sf[z] = nf[z];
-    }
+#pragma unroll 4
+    for (int z = tid; z < N; z += NT) sm[PT::slot(z)] = nat[z];
     __syncthreads();
   }
-  for (int p = threadIdx.x; p < M; p += NT) {
-    const int f = PL::freq((p % FSTEP) * RP) + (p / FSTEP) * FSTEP;
-    if (f < Nh || f >= N) {
+  for (int b = tid; b < FSTEP; b += NT) {
+    const int fb = PL::freq(b * RP);
+#pragma unroll
+    for (int j = 0; j < RP; ++j) {
+      if (BAND_CT && j >= RP / 3 && j < 2 * (RP / 3)) continue;
+      const int f = fb + j * FSTEP;
+      if (!BAND_CT && f >= Nh && f < N) continue;
       const int z = f < Nh ? f : f - Nh;
-      if constexpr (TO_PERM) {
-        po[p] = so[z];
-        pf[p] = sf[z];
-      } else {
-        so[z] = po[p];
-        sf[z] = pf[p];
-      }
+      if constexpr (TO_PERM)
+        perm[j * FSTEP + b] = sm[PT::slot(z)];
+      else
+        sm[PT::slot(z)] = perm[j * FSTEP + b];
     }
   }
+  __syncthreads();
   if constexpr (!TO_PERM) {
-    __syncthreads();
-    for (int z = threadIdx.x; z < N; z += NT) {
-      no[z] = so[z];
-      nf[z] = sf[z];
-    }
+#pragma unroll 4
+    for (int z = tid; z < N; z += NT) nat[z] = sm[PT::slot(z)];
   }
+}
+template <typename T, class PL, bool TO_PERM, int NT>
+__device__ __forceinline__ void om_perm_body(const StepArgs& a0, const Blk bk, bool om, bool fm) {
+  using C = cplx<T>;
+  const StepArgs a = member_args(a0, sizeof(C), bk.y);
+  constexpr int M = PL::M, N = 2 * M / 3;
+  extern __shared__ __align__(128) unsigned char smraw[];
+  C* sm = reinterpret_cast<C*>(smraw);
+  const int kx = bk.x;
+  if (om)
+    om_perm_column<T, PL, TO_PERM, NT>(sm, static_cast<C*>(a.om) + (size_t)kx * N,
+                                       static_cast<C*>(a.om_p) + (size_t)kx * M, threadIdx.x);
+  if (om && fm) __syncthreads();
+  if (fm)
+    om_perm_column<T, PL, TO_PERM, NT>(sm, static_cast<C*>(a.fnm1) + (size_t)kx * N,
+                                       static_cast<C*>(a.fm_p) + (size_t)kx * M, threadIdx.x);
 }
 template <typename T, class PL, bool TO_PERM>
 __global__ void __launch_bounds__(256) k_om_perm(StepArgs a0) {
-  om_perm_body<T, PL, TO_PERM, 256>(a0, hw_blk());
+  om_perm_body<T, PL, TO_PERM, 256>(a0, hw_blk(), blockIdx.z == 0, blockIdx.z == 1);
 }
 
 // k_col_inv: velocity low band -> pad -> inverse z-FFT -> U planes.  The low

@@ -38,7 +38,8 @@ struct ColKernels {
   void (*col_inv)(const StepArgs&, cudaStream_t);
   void (*twiddles)(void* tw, cudaStream_t);
   // the same pass on butterfly-major om / fnm1 (a.om_p, a.fm_p), and the
-  // conversions between that order and the natural columns
+  // conversions between that order and the natural columns (om alone under
+  // F_NO_FM_IN)
   void (*col_perm)(const StepArgs&, cudaStream_t);
   void (*to_perm)(const StepArgs&, cudaStream_t);
   void (*from_perm)(const StepArgs&, cudaStream_t);
@@ -239,13 +240,17 @@ struct ColOf {
     else
       k_col<T, PL, NT, PERM_PREF, true, false><<<grid(a), NT, smem_inv, s>>>(a);
   }
-  static constexpr size_t smem_perm = size_t(2) * (2 * PL::M / 3) * sizeof(cplx<T>);  // one om + fnm1 column
+  static constexpr size_t smem_perm = PermTile<T, PL>::smem;  // one om or fnm1 column
   static_assert(smem_perm <= kSmemLimit, "om / fnm1 column does not fit in shared memory");
+  static dim3 grid_perm(const StepArgs& a) {
+    const dim3 g = grid(a);
+    return dim3(g.x, g.y, (a.flags & F_NO_FM_IN) ? 1 : 2);
+  }
   static void to_perm(const StepArgs& a, cudaStream_t s) {
-    k_om_perm<T, PL, true><<<grid(a), 256, smem_perm, s>>>(a);
+    k_om_perm<T, PL, true><<<grid_perm(a), 256, smem_perm, s>>>(a);
   }
   static void from_perm(const StepArgs& a, cudaStream_t s) {
-    k_om_perm<T, PL, false><<<grid(a), 256, smem_perm, s>>>(a);
+    k_om_perm<T, PL, false><<<grid_perm(a), 256, smem_perm, s>>>(a);
   }
   static void col_inv(const StepArgs& a, cudaStream_t s) {
     k_col_inv<T, PL, NT><<<dim3(a.N / 2, a.members > 1 ? a.members : 1), NT, smem_inv, s>>>(a);
