@@ -19,9 +19,11 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <type_traits>
 #include <utility>
 
 #include "pal_consts.h"
+#include "pal_fixed.cuh"
 
 namespace pal {
 
@@ -45,7 +47,9 @@ template <int R, int E, int SIGN, typename C>
 __device__ __forceinline__ C twc(C a) {
   using T = decltype(a.x);
   constexpr int e = ((E % R) + R) % R;
-  if constexpr (e == 0) {
+  if constexpr (std::is_same_v<C, fxc>) {
+    return fx_twc<R, E, SIGN>(a);
+  } else if constexpr (e == 0) {
     return a;
   } else if constexpr ((4 * e) % R == 0) {
     constexpr int q = 4 * e / R;  // quarter turns
@@ -85,11 +89,19 @@ template <int SIGN, typename C> struct Dft<2, SIGN, C> {
 template <int SIGN, typename C> struct Dft<3, SIGN, C> {
   static __device__ __forceinline__ void run(C* x) {
     using T = decltype(x[0].x);
-    constexpr T h = T(0.8660254037844386467637232);  // sin(2 pi / 3)
     C t = cadd(x[1], x[2]);
     C d = csub(x[1], x[2]);
-    C m = {x[0].x - T(0.5) * t.x, x[0].y - T(0.5) * t.y};
-    C r = SIGN > 0 ? C{-h * d.y, h * d.x} : C{h * d.y, -h * d.x};
+    C m, r;
+    if constexpr (std::is_same_v<C, fxc>) {
+      constexpr long long h = TrigQ<6>::s[1];  // sin(2 pi / 3)
+      m = C{x[0].x - fx_half(t.x), x[0].y - fx_half(t.y)};
+      const C q = {fx_mulc(d.x, fx_hi(h), fx_lo(h)), fx_mulc(d.y, fx_hi(h), fx_lo(h))};
+      r = SIGN > 0 ? C{-q.y, q.x} : C{q.y, -q.x};
+    } else {
+      constexpr T h = T(0.8660254037844386467637232);  // sin(2 pi / 3)
+      m = C{x[0].x - T(0.5) * t.x, x[0].y - T(0.5) * t.y};
+      r = SIGN > 0 ? C{-h * d.y, h * d.x} : C{h * d.y, -h * d.x};
+    }
     x[0] = cadd(x[0], t);
     x[1] = cadd(m, r);
     x[2] = csub(m, r);

@@ -9,6 +9,8 @@ const pal::KernelSet* pal_kernels_f32_e(int N);
 const pal::KernelSet* pal_kernels_f32_f(int N);
 const pal::KernelSet* pal_kernels_f64_a(int N);
 const pal::KernelSet* pal_kernels_f64_b(int N);
+const pal::KernelSet* pal_kernels_f64_c(int N);
+const pal::KernelSet* pal_kernels_f64_d(int N);
 
 const pal::KernelSet* pal_kernels_f32(int N) {
   if (auto* k = pal_kernels_f32_a(N)) return k;
@@ -21,5 +23,7 @@ const pal::KernelSet* pal_kernels_f32(int N) {
 
 const pal::KernelSet* pal_kernels_f64(int N) {
   if (auto* k = pal_kernels_f64_a(N)) return k;
-  return pal_kernels_f64_b(N);
+  if (auto* k = pal_kernels_f64_b(N)) return k;
+  if (auto* k = pal_kernels_f64_c(N)) return k;
+  return pal_kernels_f64_d(N);
 }

@@ -1,42 +1,40 @@
-// FP64 candidates, N = 1536 .. 4096.
+// FP64 candidates, N = 768 .. 1536, with fixed-point transforms
+// (pal_fx_kernels.cuh).
 #include "pal_launch.cuh"
 
 using namespace pal;
 
 namespace {
+using P1152 = Plan<1152, 12, 12, 8>;
+using P1152b = Plan<1152, 8, 12, 12>;
+using P1536 = Plan<1536, 12, 16, 8>;
+using P1536b = Plan<1536, 3, 8, 8, 8>;
+using P1536c = Plan<1536, 8, 16, 12>;
+using P1536d = Plan<1536, 8, 4, 4, 12>;
 using P2304 = Plan<2304, 16, 12, 12>;
-using P3072 = Plan<3072, 16, 12, 16>;
-using P4608 = Plan<4608, 12, 24, 16>;
-using P6144 = Plan<6144, 16, 24, 16>;
-using P6144b = Plan<6144, 16, 16, 24>;
-using P6144c = Plan<6144, 8, 8, 8, 12>;
+using P2304b = Plan<2304, 4, 6, 8, 12>;
 
-const RowKernels r1536[] = {RowOf<double, P2304, 2, 256>::make("16.12.12 V2x256")};
-const ColKernels c1536[] = {ColOf<double, P2304, 256>::make("16.12.12 x256")};
-const RowKernels r2048[] = {RowOf<double, P3072, 2, 256>::make("16.12.16 V2x256"),
-                            RowOf<double, P3072, 1, 256>::make("16.12.16 V1x256")};
-const ColKernels c2048[] = {ColOf<double, P3072, 256>::make("16.12.16 x256"), ColOf<double, P3072, 128>::make("16.12.16 x128")};
-const RowKernels r3072[] = {RowOf<double, P4608, 2, 256>::make("12.24.16 V2x256")};
-const ColKernels c3072[] = {ColOf<double, P4608, 256>::make("12.24.16 x256")};
-const RowKernels r4096[] = {RowOf<double, P6144, 2, 256>::make("16.24.16 V2x256"),
-                            RowOf<double, P6144, 1, 256>::make("16.24.16 V1x256"),
-                            RowOf<double, P6144b, 1, 256>::make("16.16.24 V1x256"),
-                            RowOf<double, P6144c, 1, 256>::make("8.8.8.12 V1x256")};
-const ColKernels c4096[] = {ColOf<double, P6144, 256>::make("16.24.16 x256"), ColOf<double, P6144, 128>::make("16.24.16 x128"),
-                            ColOf<double, P6144b, 256>::make("16.16.24 x256"), ColOf<double, P6144c, 256>::make("8.8.8.12 x256")};
+const RowKernels r768[] = {RowFxOf<P1152, 2, 192>::make("12.12.8 V2x192 fx"),
+                           RowFxOf<P1152b, 2, 192>::make("8.12.12 V2x192 fx")};
+const ColKernels c768[] = {ColFxOf<P1152b, 192>::make("8.12.12 x192 fx")};
+const RowKernels r1024[] = {RowFxOf<P1536, 1, 128>::make("12.16.8 V1x128 fx"),
+                           RowFxOf<P1536b, 1, 192>::make("3.8.8.8 V1x192 fx")};
+const ColKernels c1024[] = {ColFxOf<P1536c, 192>::make("8.16.12 x192 fx"),
+                           ColFxOf<P1536d, 256>::make("8.4.4.12 x256 fx")};
+const RowKernels r1536[] = {RowFxOf<P2304b, 1, 192>::make("4.6.8.12 V1x192 fx")};
+const ColKernels c1536[] = {ColFxOf<P2304, 192>::make("16.12.12 x192 fx"),
+                           ColFxOf<P2304b, 192>::make("4.6.8.12 x192 fx")};
 
+PAL_KERNEL_SET(double, 1, 768, r768, c768)
+PAL_KERNEL_SET(double, 1, 1024, r1024, c1024)
 PAL_KERNEL_SET(double, 1, 1536, r1536, c1536)
-PAL_KERNEL_SET(double, 1, 2048, r2048, c2048)
-PAL_KERNEL_SET(double, 1, 3072, r3072, c3072)
-PAL_KERNEL_SET(double, 1, 4096, r4096, c4096)
 }  // namespace
 
 const KernelSet* pal_kernels_f64_b(int N) {
   switch (N) {
+    case 768: return &kSet768;
+    case 1024: return &kSet1024;
     case 1536: return &kSet1536;
-    case 2048: return &kSet2048;
-    case 3072: return &kSet3072;
-    case 4096: return &kSet4096;
     default: return nullptr;
   }
 }

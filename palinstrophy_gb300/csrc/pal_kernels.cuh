@@ -1673,6 +1673,49 @@ __global__ void __launch_bounds__(256) k_om_perm(StepArgs a0) {
 // band comes from `src` (reference layout (2, N, N/2), e.g. the generator's
 // uc_full) or, when src is null, from the omega -> velocity inversion of om
 // (turbo_simulator.py:1555-1585).
+// The value that k_col_inv transforms at position pos (digit-reversed) of line
+// v of column kx.
+template <typename T, class PL>
+__device__ __forceinline__ cplx<T> col_inv_value(const StepArgs& a, int kx, int v, int pos) {
+  using C = cplx<T>;
+  const int N = a.N, Nh = N >> 1;
+  const C* __restrict__ src = static_cast<const C*>(a.src);
+  const C* __restrict__ om = static_cast<const C*>(a.om) + (size_t)kx * N;
+  const int f = PL::freq(pos);
+  C val = {T(0), T(0)};
+  if (f < Nh || f >= N) {
+    const int z = f < Nh ? f : f - Nh;
+    if (a.scheme != 0) {
+      // scalar band for display (turbo_simulator.py:2639-2709): omega, or the
+      // streamfunction omega/(K2 + 1e-30); the kz = -N/2 row is left out
+      if (v == 0 && z != Nh) {
+        const C o = om[z];
+        if (a.scheme == 1) {
+          val = o;
+        } else {
+          const T gz = T(z < Nh ? z : z - N);
+          const T ik = T(1) / (T(kx) * T(kx) + gz * gz + T(1.0e-30));
+          val = C{o.x * ik, o.y * ik};
+        }
+      }
+    } else if (src != nullptr) {
+      val = src[(size_t)v * N * Nh + (size_t)z * Nh + kx];
+    } else {
+      const C o = om[z];
+      const T gz = T(z < Nh ? z : z - N);
+      const T ax = T(kx);
+      if (kx >= 1) {
+        const T ik = T(1) / (ax * ax + gz * gz);
+        const C t = {o.x * ik, o.y * ik};
+        val = (v == 0) ? C{t.y * gz, -t.x * gz} : C{-t.y * ax, t.x * ax};
+      } else if (v == 0 && z >= 1) {
+        const T ig = T(1) / gz;
+        val = C{o.y * ig, -o.x * ig};
+      }
+    }
+  }
+  return val;
+}
 template <typename T, class PL, int NT>
 __global__ void __launch_bounds__(NT) k_col_inv(StepArgs a0) {
   using C = cplx<T>;
@@ -1683,48 +1726,8 @@ __global__ void __launch_bounds__(NT) k_col_inv(StepArgs a0) {
   constexpr int V = 2;
   const int tid = threadIdx.x;
   const int kx = blockIdx.x;
-  const int N = a.N, Nh = N >> 1;
   const C* __restrict__ tw = static_cast<const C*>(a.tw);
-  const C* __restrict__ src = static_cast<const C*>(a.src);
-  const C* __restrict__ om = static_cast<const C*>(a.om) + (size_t)kx * N;
-  for (int w = tid; w < V * M; w += NT) {
-    const int v = w & 1;
-    const int pos = w >> 1;
-    const int f = PL::freq(pos);
-    C val = {T(0), T(0)};
-    if (f < Nh || f >= N) {
-      const int z = f < Nh ? f : f - Nh;
-      if (a.scheme != 0) {
-        // scalar band for display (turbo_simulator.py:2639-2709): omega, or the
-        // streamfunction omega/(K2 + 1e-30); the kz = -N/2 row is left out
-        if (v == 0 && z != Nh) {
-          const C o = om[z];
-          if (a.scheme == 1) {
-            val = o;
-          } else {
-            const T gz = T(z < Nh ? z : z - N);
-            const T ik = T(1) / (T(kx) * T(kx) + gz * gz + T(1.0e-30));
-            val = C{o.x * ik, o.y * ik};
-          }
-        }
-      } else if (src != nullptr) {
-        val = src[(size_t)v * N * Nh + (size_t)z * Nh + kx];
-      } else {
-        const C o = om[z];
-        const T gz = T(z < Nh ? z : z - N);
-        const T ax = T(kx);
-        if (kx >= 1) {
-          const T ik = T(1) / (ax * ax + gz * gz);
-          const C t = {o.x * ik, o.y * ik};
-          val = (v == 0) ? C{t.y * gz, -t.x * gz} : C{-t.y * ax, t.x * ax};
-        } else if (v == 0 && z >= 1) {
-          const T ig = T(1) / gz;
-          val = C{o.y * ig, -o.x * ig};
-        }
-      }
-    }
-    sm[PL::phys(pos) * V + v] = val;
-  }
+  for (int w = tid; w < V * M; w += NT) sm[PL::phys(w >> 1) * V + (w & 1)] = col_inv_value<T, PL>(a, kx, w & 1, w >> 1);
   __syncthreads();
   dit_range<T, PL, V, NT, +1, PL::NP - 1, 0>(sm, tw, tid);
   C* __restrict__ w0 = static_cast<C*>(a.w0);

@@ -10,6 +10,7 @@
 #include <cstdlib>
 
 #include "pal_adjoint.cuh"
+#include "pal_fx_kernels.cuh"
 #include "pal_kernels.cuh"
 
 namespace pal {
@@ -267,6 +268,83 @@ struct ColOf {
   static constexpr ColKernels make(const char* name) {
     return ColKernels{name,    NT,     smem,     PL::TW_TOTAL,          configure, col,
                       col_inv, launch_twiddles<T, PL>, col_perm, to_perm, from_perm, blocks_per_sm, TMA, PL::RP};
+  }
+};
+
+// FP64 passes with fixed-point transforms (pal_fx_kernels.cuh).  MINB > 0 caps
+// the registers so that MINB blocks share an SM.
+template <class PL>
+void launch_twiddles_fx(void* tw, cudaStream_t s) {
+  using FP = FxPlan<PL>;
+  if (FP::TW_TOTAL > 0) k_twiddles_fx<FP><<<(FP::TW_TOTAL + 127) / 128, 128, 0, s>>>(static_cast<int4*>(tw));
+}
+
+template <class K>
+cudaError_t set_tile_smem(K kernel, size_t smem) {
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess && smem >= kLargeTile)
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
+  return e;
+}
+
+template <class PL, int V, int NT, int MINB = 0>
+struct RowFxOf {
+  using FP = FxPlan<PL>;
+  static constexpr size_t smem = size_t(PL::PADM) * V * sizeof(fxc);
+  static_assert(smem <= kSmemLimit && PL::M % V == 0 && NT % 32 == 0, "row tile, whole warps");
+  static cudaError_t configure() {
+    cudaError_t e = set_tile_smem(k_row_fx<FP, V, NT, MINB>, smem);
+    return e == cudaSuccess ? set_tile_smem(k_phys_fx<FP, V, NT>, smem) : e;
+  }
+  static dim3 grid(const StepArgs& a) { return dim3(PL::M / V, a.members > 1 ? a.members : 1); }
+  static void row(const StepArgs& a, cudaStream_t s) { k_row_fx<FP, V, NT, MINB><<<grid(a), NT, smem, s>>>(a); }
+  static void phys(const StepArgs& a, cudaStream_t s) { k_phys_fx<FP, V, NT><<<grid(a), NT, smem, s>>>(a); }
+  static int blocks_per_sm() {
+    int n = 0;
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_row_fx<FP, V, NT, MINB>, NT, smem) == cudaSuccess ? n : -1;
+  }
+  static constexpr RowKernels make(const char* name) {
+    return RowKernels{name, V, NT, false, smem, FP::TW_TOTAL, configure, row, phys, launch_twiddles_fx<PL>, blocks_per_sm};
+  }
+};
+
+template <class PL, int NT, int MINB = 0>
+struct ColFxOf {
+  using FP = FxPlan<PL>;
+  static constexpr size_t smem = size_t(PL::PADM) * 2 * sizeof(fxc);
+  static constexpr size_t smem_perm = PermTile<double, PL>::smem;
+  static_assert(smem <= kSmemLimit && smem_perm <= kSmemLimit && NT % 32 == 0, "column tile, whole warps");
+  static cudaError_t configure() {
+    cudaError_t e = set_tile_smem(k_col_fx<FP, NT, false, MINB>, smem);
+    if (e == cudaSuccess) e = set_tile_smem(k_col_fx<FP, NT, true, MINB>, smem);
+    if (e == cudaSuccess) e = set_tile_smem(k_col_inv_fx<FP, NT>, smem);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(k_om_perm<double, PL, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_perm);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(k_om_perm<double, PL, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_perm);
+    return e;
+  }
+  static dim3 grid(const StepArgs& a) { return dim3(a.N / 2, a.members > 1 ? a.members : 1); }
+  static dim3 grid_perm(const StepArgs& a) {
+    const dim3 g = grid(a);
+    return dim3(g.x, g.y, (a.flags & F_NO_FM_IN) ? 1 : 2);
+  }
+  static void col(const StepArgs& a, cudaStream_t s) { k_col_fx<FP, NT, false, MINB><<<grid(a), NT, smem, s>>>(a); }
+  static void col_perm(const StepArgs& a, cudaStream_t s) { k_col_fx<FP, NT, true, MINB><<<grid(a), NT, smem, s>>>(a); }
+  static void col_inv(const StepArgs& a, cudaStream_t s) { k_col_inv_fx<FP, NT><<<grid(a), NT, smem, s>>>(a); }
+  static void to_perm(const StepArgs& a, cudaStream_t s) {
+    k_om_perm<double, PL, true><<<grid_perm(a), 256, smem_perm, s>>>(a);
+  }
+  static void from_perm(const StepArgs& a, cudaStream_t s) {
+    k_om_perm<double, PL, false><<<grid_perm(a), 256, smem_perm, s>>>(a);
+  }
+  static int blocks_per_sm() {
+    int n = 0;
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_col_fx<FP, NT, true, MINB>, NT, smem) == cudaSuccess ? n : -1;
+  }
+  static constexpr ColKernels make(const char* name) {
+    return ColKernels{name,     NT,      smem,      FP::TW_TOTAL,  configure, col, col_inv, launch_twiddles_fx<PL>,
+                      col_perm, to_perm, from_perm, blocks_per_sm, false,     PL::RP};
   }
 };
 

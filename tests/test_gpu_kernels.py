@@ -34,3 +34,126 @@ def test_methods_alternate(N):
     assert do.rel_l2(S.om2, F.om2()) <= 1e-12
     assert do.rel_l2(S.fnm1, F.fnm1()) <= 1e-10
     F.close()
+
+
+def _long_double_step(om, dt, nu):
+    """u, fn and om2 of one CNAB2 step (cnm1 = 0) in NumPy's long double."""
+    import scipy.fft as sf
+
+    L = np.longdouble
+    N = om.shape[0]
+    nh, M = N // 2, 3 * N // 2
+    kx = np.arange(nh).astype(L)[None, :]
+    kz = np.where(np.arange(N) < nh, np.arange(N), np.arange(N) - N).astype(L)[:, None]
+    k2 = kx * kx + kz * kz
+    inv = 1 / np.where(k2 > 0, k2, 1)
+    om = om.astype(np.clongdouble)
+
+    def phys(b):
+        X = np.zeros((M, M // 2 + 1), np.clongdouble)
+        X[:nh, :nh], X[N:, :nh] = b[:nh], b[nh:]
+        return sf.irfft2(X, s=(M, M), norm="forward")
+
+    def gather(s):
+        return np.concatenate((s[:nh, :nh], s[N:, :nh]))
+
+    u, v = phys(-1j * kz * inv * om), phys(1j * kx * inv * om)
+    fn = (kz * kx * gather(sf.rfft2(u * u - v * v)) + (kz * kz - kx * kx) * gather(sf.rfft2(u * v))) / L(M) ** 2
+    fn[nh] = 0
+    h = L(nu) * L(dt) / 2
+    return u, fn, ((1 - k2 * h) * om + L(dt) * fn) / (1 + k2 * h)
+
+
+def _spectrum(N, kind):
+    rng = np.random.default_rng(N)
+    nh = N // 2
+    k = np.hypot(np.arange(nh)[None, :], np.fft.fftfreq(N, 1.0 / N)[:, None])
+    k[0, 0] = 1.0
+    om = np.exp(2j * np.pi * rng.random((N, nh)))
+    om *= {"k-1": 1.0 / k, "steep": np.exp(-0.5 * k), "white": 1.0}[kind]
+    om[nh] = om[0, 0] = 0.0
+    om[nh + 1:, 0] = np.conj(om[1:nh, 0][::-1])
+    return om
+
+
+@pytest.mark.parametrize("kind", ["k-1", "steep", "white"])
+@pytest.mark.parametrize("N", [32, 64, 128, 256, 384])
+def test_fixed_point_transforms_are_no_worse_than_fp64(N, kind):
+    """The FP64 form's block fixed-point transforms against long double: the
+    velocity and the nonlinear term are as close to it as an FP64 transform's
+    (the oracle's, in NumPy / SciPy double), the update as close as FP64 rounds."""
+    from palinstrophy_gb300.turbo_simulator import Field
+
+    dt, nu = 1e-3, 1e-3
+    om = _spectrum(N, kind)
+    u, fn, on = _long_double_step(om, dt, nu)
+    F = Field(N, "fp64", 1e3, 0.3)
+    F.set_state(om)
+    F.set_scalars(dt=dt, cn=1.0, cnm1=0.0, visc=nu, cflnum=0.3)
+    F.step2a()
+    gu = F.ur(0)
+    F.step("CNAB2", 1)
+    kx = np.arange(N // 2)[None, :]
+    kz = np.where(np.arange(N) < N // 2, np.arange(N), np.arange(N) - N)[:, None]
+    k2 = np.where(kx * kx + kz * kz > 0, kx * kx + kz * kz, 1)
+    S = do.OracleState(N, om, np.stack([-1j * kz * om / k2, 1j * kx * om / k2]), nu, 0.3)
+    S.dt, S.cn, S.cnm1 = dt, 1.0, 0.0
+    do.step2a(S)
+
+    def err(x, ref):
+        return float(np.linalg.norm((x.astype(ref.dtype) - ref).ravel().astype(np.complex128))
+                     / np.linalg.norm(ref.ravel().astype(np.complex128)))
+
+    ou = err(S.ur_full[0], u)
+    do.cnab2(S)
+    # a transform rounds at least once per pass: never asked to be below 2 eps
+    eps = np.finfo(np.float64).eps
+    assert err(gu, u) <= max(ou, 2 * eps)
+    assert err(F.fnm1(), fn) <= max(err(S.fnm1, fn), 2 * eps)
+    assert err(F.om2(), on) <= max(err(S.om2, on), 2 * eps)
+    F.close()
+
+
+@pytest.mark.parametrize("scale", [1e-290, 1e-160, 1e-30, 1e30, 1e140])
+@pytest.mark.parametrize("N", [32, 256])
+def test_fixed_point_follows_the_field_scale(N, scale):
+    """A power-of-two scaled field gives the scaled velocity exactly (as long as
+    no stored value is subnormal)."""
+    from palinstrophy_gb300.turbo_simulator import Field
+
+    s = 2.0 ** np.round(np.log2(scale))
+    om = _spectrum(N, "k-1")
+    got = []
+    for f in (1.0, s):
+        F = Field(N, "fp64", 1e3, 0.3)
+        F.set_state(om * f)
+        F.step2a()
+        got.append((F.ur(0), F.ur(1)))
+        F.close()
+    for a, b in zip(*got):
+        assert np.array_equal(a * s, b)
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+@pytest.mark.parametrize("N", [32, 512])
+def test_fixed_point_non_finite_fields(N, bad):
+    """A NaN or an infinity in the field reaches every value of the next one and
+    the diagnostics report it; a zero field stays zero."""
+    from palinstrophy_gb300.turbo_simulator import Field
+
+    om = _spectrum(N, "k-1")
+    om[3, 2] = bad
+    F = Field(N, "fp64", 1e3, 0.3)
+    F.set_state(om)
+    F.set_scalars(dt=1e-3, visc=1e-3)
+    F.step("CNAB2", 2)
+    # the nonlinear term of the row kz = -N/2 is zero by definition
+    assert not np.isfinite(np.delete(F.om2(), N // 2, axis=0)[:, 1:]).any()
+    assert F.diagnostics()["nonfinite"] == 1
+    F.close()
+    F = Field(N, "fp64", 1e3, 0.3)
+    F.set_state(np.zeros_like(om))
+    F.set_scalars(dt=1e-3, visc=1e-3)
+    F.step("LS_IMEX_RK3", 2)
+    assert not F.om2().any() and not F.ur(0).any()
+    F.close()
