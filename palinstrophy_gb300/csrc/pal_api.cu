@@ -55,6 +55,8 @@ struct pal_handle {
   void *stage = nullptr, *phys = nullptr;
   void *vis_w = nullptr;      // two scratch work planes for display transforms
   void *vis_phys = nullptr;   // three physical planes (u|scalar, v, |u|)
+  void *spec = nullptr, *spec_host = nullptr;  // energy-spectrum bins (device, pinned host), grown on demand
+  size_t spec_bytes = 0;
   DevScalars* sc = nullptr;
   DevScalars* sc_host = nullptr;  // pinned mirror
   double* part = nullptr;
@@ -507,7 +509,8 @@ int pal_create(int N, int precision, double Re, double cfl, pal_handle** out) {
   int sms = 0, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  h->spectral_blocks = std::max(1, std::min(4 * sms, (int)(((size_t)N * h->Nh + 255) / 256)));
+  // two blocks per SM: a block's FP64 reduction tree costs as much as ten modes per thread
+  h->spectral_blocks = std::max(1, std::min(2 * sms, (int)(((size_t)N * h->Nh + 255) / 256)));
   const size_t part_n = (size_t)std::max(h->M, std::max(1024, h->spectral_blocks)) * 5;
   void** bufs[] = {&h->w0, &h->w1, &h->om, &h->fnm1, &h->stage, &h->tw_row, &h->tw_col, &h->om_p};
   const size_t sizes[] = {plane_w + pal::kPlaneSlack, plane_w + pal::kPlaneSlack, plane_om, plane_om, 2 * plane_om,
@@ -547,9 +550,11 @@ int pal_destroy(pal_handle* h) {
   for (auto& kv : h->step_graphs) cudaGraphExecDestroy(kv.second);
   h->step_graphs.clear();
   void* bufs[] = {h->w0,     h->w1,   h->om,   h->fnm1, h->stage, h->tw_row,   h->tw_col,
-                  h->phys,   h->sc,   h->part, h->vis_w, h->vis_phys, h->om_p};
+                  h->phys,   h->sc,   h->part, h->vis_w, h->vis_phys, h->om_p,
+                  h->spec};
   for (void* b : bufs)
     if (b) cudaFree(b);
+  if (h->spec_host) cudaFreeHost(h->spec_host);
   if (h->sc_host) cudaFreeHost(h->sc_host);
   if (h->stream) cudaStreamDestroy(h->stream);
   delete h;
@@ -816,18 +821,28 @@ int pal_energy_spectrum(pal_handle* h, int nbins, double r_max, double k_nyq, do
   if (nbins <= 0 || !(r_max > 0.0) || !(k_nyq > 0.0) || !esum || !count)
     return fail(h, PAL_ERR_INVALID, "bad spectrum arguments");
   if (h->state == ST_EMPTY) return fail(h, PAL_ERR_STATE, "no spectral state set");
-  double* d_e = nullptr;
-  PAL_CK(h, cudaMallocAsync(reinterpret_cast<void**>(&d_e), (size_t)nbins * (sizeof(double) + sizeof(int)),
-                            h->stream));
+  // energies, counts and bin edges in one device buffer of the handle, the first
+  // two read back with one copy through its pinned mirror
+  const size_t out_bytes = (size_t)nbins * (sizeof(double) + sizeof(int));
+  const size_t bytes = out_bytes + ((size_t)nbins + 1) * sizeof(int);
+  if (h->spec_bytes < bytes) {
+    if (h->spec) cudaFree(h->spec);
+    if (h->spec_host) cudaFreeHost(h->spec_host);
+    h->spec = h->spec_host = nullptr;
+    h->spec_bytes = 0;
+    PAL_CK(h, cudaMalloc(&h->spec, bytes));
+    PAL_CK(h, cudaMallocHost(&h->spec_host, out_bytes));
+    h->spec_bytes = bytes;
+  }
+  double* d_e = static_cast<double*>(h->spec);
   int* d_c = reinterpret_cast<int*>(d_e + nbins);
   const double scale = (double)h->M * (double)h->M;
-  h->ks->spectrum(h->om, h->N, nbins, r_max, k_nyq, scale * scale, d_e, d_c, h->stream);
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaMemcpyAsync(esum, d_e, nbins * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(count, d_c, nbins * sizeof(int), cudaMemcpyDeviceToHost, h->stream);
-  cudaFreeAsync(d_e, h->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-  if (e != cudaSuccess) return cuda_fail(h, e, "energy spectrum");
+  h->ks->spectrum(h->om, h->N, nbins, r_max, k_nyq, scale * scale, d_e, d_c, d_c + nbins, h->stream);
+  PAL_LAUNCHED(h, "energy spectrum");
+  PAL_CK(h, cudaMemcpyAsync(h->spec_host, h->spec, out_bytes, cudaMemcpyDeviceToHost, h->stream));
+  PAL_CK(h, cudaStreamSynchronize(h->stream));
+  std::memcpy(esum, h->spec_host, nbins * sizeof(double));
+  std::memcpy(count, static_cast<char*>(h->spec_host) + nbins * sizeof(double), nbins * sizeof(int));
   return PAL_OK;
 }
 

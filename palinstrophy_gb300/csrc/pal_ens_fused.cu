@@ -42,6 +42,7 @@ struct FusedSize {
   }
   template <int NT>
   static __device__ __forceinline__ void phys(const StepArgs& a, Blk bk) {
+    static_assert(size_t(PLR::PADM) * VR * sizeof(float2) >= size_t(2) * NT * sizeof(double), "phys_body's tile");
     phys_body<float, PLR, VR, NT>(a, bk);
   }
   template <int NT, bool TO>

@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(NT, MINB) k_row_fx(StepArgs a0) {
 }
 
 // k_phys in fixed point: U-state rows -> physical u, v (statistics, optional
-// plane store).
+// plane store), tiles and statistics as phys_body.
 template <class PL, int V, int NT>
 __global__ void __launch_bounds__(NT) k_phys_fx(StepArgs a0) {
   const Blk bk = hw_blk();
@@ -334,37 +334,43 @@ __global__ void __launch_bounds__(NT) k_phys_fx(StepArgs a0) {
   __shared__ FxWords ws;
   fxc* sm = reinterpret_cast<fxc*>(smraw);
   constexpr int M = PL::M;
+  static_assert(size_t(PL::PADM) * V * sizeof(fxc) >= size_t(2) * NT * sizeof(double), "finish_stats' sums fit in the tile");
   const int tid = threadIdx.x;
-  const int z0 = bk.x * V;
-  FxScale sc;
-  fx_rows_inverse<PL, V, NT>(a.w0, a.w1, sm, static_cast<const int4*>(a.tw), z0, tid, &ws, sc);
-  double acc = 0.0, comp = 0.0;
-  unsigned long long top = 0;
+  double mx = 0.0, acc = 0.0, comp = 0.0;
   double* __restrict__ ph = static_cast<double*>(a.phys);
   const bool store = (a.flags & F_PHYS) != 0;
   const bool diag = (a.flags & F_DIAG) != 0;
-  for (int w = tid; w < V * M; w += NT) {
-    const int v = w % V;
-    const int pos = w / V;
-    const fxc q = sm[PL::phys(pos) * V + v];
-    const double x = fx_value(q.x, sc), y = fx_value(q.y, sc);
-    top = max(top, fx_speed(q));
-    const double e = fma(x, x, y * y);
-    if (diag)
-      csum_add(acc, comp, e);
-    else
-      acc += e;  // finiteness check only
-    if (store) {
-      const int n = PL::freq(pos);
-      ph[(size_t)(z0 + v) * M + n] = x;
-      ph[(size_t)M * M + (size_t)(z0 + v) * M + n] = y;
+  SquareSum quad;
+  for (int tile = bk.x; tile < M / V; tile += bk.nx) {
+    const int z0 = tile * V;
+    FxScale sc;
+    fx_rows_inverse<PL, V, NT>(a.w0, a.w1, sm, static_cast<const int4*>(a.tw), z0, tid, &ws, sc);
+    unsigned long long top = 0;
+    for (int w = tid; w < V * M; w += NT) {
+      const int v = w % V;
+      const int pos = w / V;
+      const fxc q = sm[PL::phys(pos) * V + v];
+      const double x = fx_value(q.x, sc), y = fx_value(q.y, sc);
+      top = max(top, fx_speed(q));
+      if (diag)
+        quad.add(x, y, acc, comp);
+      else
+        acc = fma(x, x, fma(y, y, acc));  // finiteness check only
+      if (store) {
+        const int n = PL::freq(pos);
+        ph[(size_t)(z0 + v) * M + n] = x;
+        ph[(size_t)M * M + (size_t)(z0 + v) * M + n] = y;
+      }
     }
+    mx = fmax(mx, fx_speed_value(top, sc));
+    __syncthreads();  // the tile and its words are free
   }
-  const double mx = fx_speed_value(top, sc);
-  if (diag)
-    finish_stats<NT, true>(a, mx, acc, comp, M, tid, bk);
-  else
+  if (diag) {
+    quad.flush(acc, comp);
+    finish_stats<NT, true>(a, mx, acc, comp, M, tid, bk, reinterpret_cast<double*>(smraw));
+  } else {
     finish_stats<NT, false>(a, mx, acc, 0.0, M, tid, bk);
+  }
 }
 
 // 1 / d by two steps of Newton's iteration from the hardware's reciprocal

@@ -232,47 +232,82 @@ __device__ __forceinline__ void csum_add(double& s, double& c, double x) {
   s = t;
 }
 
-// Block-wide compensated sum of K pairs (s, c): every level of the tree adds
-// the s parts with TwoSum and the c parts plainly.  Threads 0..31 hold s + c
-// in s on return.
+// A float in FP64 without the FP64 pipe: its bits, rebiased (the pipe's own
+// conversion for zeros, subnormals, infinities and NaN).
+__device__ __forceinline__ double widen(float x) {
+  const unsigned b = __float_as_uint(x), e = b & 0x7f800000u;
+  if (e == 0u || e == 0x7f800000u) return double(x);
+  return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + (896u << 20))), (int)(b << 29));
+}
+__device__ __forceinline__ double widen(double x) { return x; }
+
+// csum_add for s, x >= 0 (no NaN ordering is needed: a NaN stays one): the
+// larger operand is found on the bit patterns, and then Fast2Sum's four FP64
+// instructions do what TwoSum needs seven for.
+__device__ __forceinline__ void csum_add_pos(double& s, double& c, double x) {
+  const long long is = __double_as_longlong(s), ix = __double_as_longlong(x);
+  const double hi = __longlong_as_double(max(is, ix)), lo = __longlong_as_double(min(is, ix));
+  s = hi + lo;
+  c += lo - (s - hi);
+}
+
+// Block-wide compensated sum of K pairs (s, c), in red (2 K NT doubles): the
+// pairs cross shared memory and warp q alone adds those of sum q, the s parts
+// with TwoSum and the c parts plainly -- 8 FP64 instructions an addition, on a
+// pipe where every warp-wide instruction takes 64 cycles, so a shuffle tree in
+// every warp cost four times as much.  Every thread holds s + c in s on return.
 template <int NT, int K>
-__device__ __forceinline__ void block_csum(double (&s)[K], double (&c)[K], double* red /* 2*K*NT/32 */, int tid) {
+__device__ __forceinline__ void block_csum(double (&s)[K], double (&c)[K], double* red, int tid) {
+  static_assert(NT % 32 == 0 && K <= (NT + 31) / 32, "one warp per sum");
 #pragma unroll
   for (int q = 0; q < K; ++q) {
+    red[2 * q * NT + tid] = s[q];
+    red[(2 * q + 1) * NT + tid] = c[q];
+  }
+  __syncthreads();
+  double ss = 0.0, cc = 0.0;
+  const int q = tid >> 5;
+  if (q < K) {
+    for (int t = tid & 31; t < NT; t += 32) {
+      csum_add(ss, cc, red[2 * q * NT + t]);
+      cc += red[(2 * q + 1) * NT + t];
+    }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
-      const double so = __shfl_xor_sync(0xffffffffu, s[q], off);
-      const double co = __shfl_xor_sync(0xffffffffu, c[q], off);
-      csum_add(s[q], c[q], so);
-      c[q] += co;
+      const double so = __shfl_xor_sync(0xffffffffu, ss, off);
+      const double co = __shfl_xor_sync(0xffffffffu, cc, off);
+      csum_add(ss, cc, so);
+      cc += co;
     }
   }
-  constexpr int NW = NT / 32;
-  if ((tid & 31) == 0) {
+  __syncthreads();
+  if (q < K && (tid & 31) == 0) red[q] = ss + cc;
+  __syncthreads();
 #pragma unroll
-    for (int q = 0; q < K; ++q) {
-      red[(2 * q) * NW + (tid >> 5)] = s[q];
-      red[(2 * q + 1) * NW + (tid >> 5)] = c[q];
-    }
+  for (int r = 0; r < K; ++r) {
+    s[r] = red[r];
+    c[r] = 0.0;
   }
+  __syncthreads();
+}
+
+// The block's maximum of values >= 0 (ordered as their bit patterns, so the
+// FP64 pipe is not needed); every thread of the first warp holds it on return.
+template <int NT>
+__device__ __forceinline__ double block_max_pos(double m, double* red, int tid) {
+  long long b = __double_as_longlong(m);
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) b = max(b, __shfl_xor_sync(0xffffffffu, b, off));
+  constexpr int NW = NT / 32;
+  if ((tid & 31) == 0) red[tid >> 5] = __longlong_as_double(b);
   __syncthreads();
   if (tid < 32) {
+    b = tid < NW ? __double_as_longlong(red[tid]) : 0;
 #pragma unroll
-    for (int q = 0; q < K; ++q) {
-      double ss = tid < NW ? red[(2 * q) * NW + tid] : 0.0;
-      double cc = tid < NW ? red[(2 * q + 1) * NW + tid] : 0.0;
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) {
-        const double so = __shfl_xor_sync(0xffffffffu, ss, off);
-        const double co = __shfl_xor_sync(0xffffffffu, cc, off);
-        csum_add(ss, cc, so);
-        cc += co;
-      }
-      s[q] = ss + cc;
-      c[q] = 0.0;
-    }
+    for (int off = 16; off > 0; off >>= 1) b = max(b, __shfl_xor_sync(0xffffffffu, b, off));
   }
   __syncthreads();
+  return __longlong_as_double(b);
 }
 
 // Returns true in every thread of the block that finished last of the nx
@@ -303,13 +338,16 @@ __device__ __forceinline__ bool last_block(unsigned int* counter, int tid) {
 // diagnostic sum); without it the sum is a plain FP64 tree, enough for the
 // finiteness check of the NEXTDT statistics and far cheaper in FP64 issue slots,
 // which matters for small tiles that take the statistics every step.
+// `wide`: 2 NT doubles of shared memory for the compensated sum (a tile that is
+// no longer needed).
 template <int NT, bool COMP>
-__device__ void finish_stats(const StepArgs& a, double mx, double sum, double comp, int M, int tid, const Blk& bk) {
+__device__ void finish_stats(const StepArgs& a, double mx, double sum, double comp, int M, int tid, const Blk& bk,
+                             double* wide = nullptr) {
   __shared__ double red[2 * (NT / 32)];
   double s1[1] = {sum}, c1[1] = {comp};
   if constexpr (COMP) {
-    mx = block_max<NT>(mx, red, tid);
-    block_csum<NT, 1>(s1, c1, red, tid);
+    mx = block_max_pos<NT>(mx, red, tid);
+    block_csum<NT, 1>(s1, c1, wide, tid);
   } else {
     block_maxsum<NT>(mx, s1[0], red, tid);
   }
@@ -329,8 +367,8 @@ __device__ void finish_stats(const StepArgs& a, double mx, double sum, double co
       s2[0] += __ldcg(a.part + 2 * q + 1);
   }
   if constexpr (COMP) {
-    m2 = block_max<NT>(m2, red, tid);
-    block_csum<NT, 1>(s2, c2, red, tid);
+    m2 = block_max_pos<NT>(m2, red, tid);
+    block_csum<NT, 1>(s2, c2, wide, tid);
   } else {
     block_maxsum<NT>(m2, s2[0], red, tid);
   }
@@ -938,7 +976,28 @@ __global__ void __launch_bounds__(NT, (PF & 16) ? row_tiles_per_sm<T, PL, V>() :
   row_body<T, PL, V, NT, PF>(a0, maps, hw_blk());
 }
 
-// k_phys: U-state rows -> physical u, v (statistics, optional plane store).
+// The diagnostic sum of u^2 + v^2 of one thread: the squares of four points run
+// into one FP64 chain of fused multiply-adds, and the chain's value is added to
+// the compensated sum.  The diagnostic k_phys is bound by the FP64 pipe: 5 FP64
+// instructions a point (conversions included) where a TwoSum per point took 11;
+// N=2048 FP32 295 us before, 173 now.
+struct SquareSum {
+  double s = 0.0;
+  int n = 0;
+  __device__ __forceinline__ void add(double u, double v, double& acc, double& comp) {
+    s = fma(u, u, fma(v, v, s));
+    if (++n == 4) flush(acc, comp);
+  }
+  __device__ __forceinline__ void flush(double& acc, double& comp) {
+    csum_add_pos(acc, comp, s);
+    s = 0.0;
+    n = 0;
+  }
+};
+
+// k_phys: U-state rows -> physical u, v (statistics, optional plane store).  A
+// block takes every bk.nx-th of the M / V tiles and reduces its statistics once.
+// Dynamic shared memory: the tile, at least 2 NT doubles (finish_stats).
 template <typename T, class PL, int V, int NT>
 __device__ __forceinline__ void phys_body(const StepArgs& a0, const Blk bk) {
   using C = cplx<T>;
@@ -947,36 +1006,41 @@ __device__ __forceinline__ void phys_body(const StepArgs& a0, const Blk bk) {
   C* sm = reinterpret_cast<C*>(smraw);
   constexpr int M = PL::M;
   const int tid = threadIdx.x;
-  const int z0 = bk.x * V;
   const C* __restrict__ tw = static_cast<const C*>(a.tw);
-  row_first_pass<T, PL, V, NT>(a, sm, z0, tid);
-  dif_range<T, PL, V, NT, +1, 1, PL::NP>(sm, tw, tid);
   T mx = T(0), accp = T(0);
   double acc = 0.0, comp = 0.0;  // F_DIAG: compensated FP64 sum of u^2 + v^2
   T* __restrict__ ph = static_cast<T*>(a.phys);
   const bool store = (a.flags & F_PHYS) != 0;
   const bool diag = (a.flags & F_DIAG) != 0;
-  for (int w = tid; w < V * M; w += NT) {
-    const int v = w % V;
-    const int pos = w / V;
-    const C val = sm[PL::phys(pos) * V + v];
-    mx = fmax(mx, fabs(val.x) + fabs(val.y));
-    if (diag) {
-      const double du = double(val.x), dq = double(val.y);
-      csum_add(acc, comp, fma(du, du, dq * dq));
-    } else {
-      accp = fma(val.x, val.x, fma(val.y, val.y, accp));  // finiteness check only
+  SquareSum quad;
+  for (int tile = bk.x; tile < M / V; tile += bk.nx) {
+    const int z0 = tile * V;
+    row_first_pass<T, PL, V, NT>(a, sm, z0, tid);
+    dif_range<T, PL, V, NT, +1, 1, PL::NP>(sm, tw, tid);
+    for (int w = tid; w < V * M; w += NT) {
+      const int v = w % V;
+      const int pos = w / V;
+      const C val = sm[PL::phys(pos) * V + v];
+      mx = fmax(mx, fabs(val.x) + fabs(val.y));
+      if (diag) {
+        quad.add(widen(val.x), widen(val.y), acc, comp);
+      } else {
+        accp = fma(val.x, val.x, fma(val.y, val.y, accp));  // finiteness check only
+      }
+      if (store) {
+        const int n = PL::freq(pos);
+        ph[(size_t)(z0 + v) * M + n] = val.x;
+        ph[(size_t)M * M + (size_t)(z0 + v) * M + n] = val.y;
+      }
     }
-    if (store) {
-      const int n = PL::freq(pos);
-      ph[(size_t)(z0 + v) * M + n] = val.x;
-      ph[(size_t)M * M + (size_t)(z0 + v) * M + n] = val.y;
-    }
+    __syncthreads();  // the tile is free
   }
-  if (diag)
-    finish_stats<NT, true>(a, double(mx), acc, comp, M, tid, bk);
-  else
+  if (diag) {
+    quad.flush(acc, comp);
+    finish_stats<NT, true>(a, double(mx), acc, comp, M, tid, bk, reinterpret_cast<double*>(smraw));
+  } else {
     finish_stats<NT, false>(a, double(mx), double(accp), 0.0, M, tid, bk);
+  }
 }
 template <typename T, class PL, int V, int NT>
 __global__ void __launch_bounds__(NT) k_phys(StepArgs a0) {
@@ -1740,41 +1804,66 @@ __global__ void __launch_bounds__(NT) k_col_inv(StepArgs a0) {
 }
 
 // --------------------------------------------------------------------------
+// isfinite without an FP64 comparison.
+__device__ __forceinline__ bool finite_bits(double x) { return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000; }
+
+// 1 / sqrt(x) for an integer x >= 1: Householder's third-order step from the
+// float estimate (relative error 2^-22 leaves 2^-64, below FP64's rounding).
+__device__ __forceinline__ double int_rsqrt(double x, int ix) {
+  const unsigned b = __float_as_uint(rsqrtf((float)ix));  // as a double: the float's bits, rebiased
+  const double y = __hiloint2double((int)((b >> 3) + (896u << 20)), (int)(b << 29));
+  const double e = fma(-(x * y), y, 1.0);
+  return fma(y, e * fma(e, 0.375, 0.5), y);
+}
+
 // Spectral sums over om [kx][z]: E = sum w |om|^2/K2, Lsum = sum w |om|^2/K2^1.5,
 // Z = sum w |om|^2 (minus the (0,0) mode), P = sum w K2 |om|^2, with the
 // rfft weights w = [1, 2, ..., 2, 1] of turbo_simulator.py:778-781 and
-// turbo_main.py:2040-2044.
+// turbo_main.py:2040-2044.  Bound by the FP64 pipe, so a thread takes the modes
+// kz and -kz together (one K2, one reciprocal root, one compensated addition
+// for both) and no division or square root: 36 FP64 instructions for two modes
+// where one took about 75.  N=2048: 421 us before, 98 now.
 template <typename T, int NT>
 __global__ void __launch_bounds__(NT) k_spectral(StepArgs a0) {
   using C = cplx<T>;
   const StepArgs a = member_args(a0, sizeof(C));
   const C* __restrict__ om = static_cast<const C*>(a.om);
   const int N = a.N, Nh = N >> 1;
-  const long long total = (long long)N * Nh;
+  const int total = (Nh + 1) * Nh;  // kz = 0 .. N/2 (row N/2 holds -N/2) of every kx
   const int tid = threadIdx.x;
   // compensated FP64 sums: E, L numerator, Z (all modes), P, and the (0,0) mode
   double s[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, c[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
   int bad = 0;
-  for (long long idx = (long long)blockIdx.x * NT + tid; idx < total; idx += (long long)gridDim.x * NT) {
-    const int kx = int(idx / N);
-    const int z = int(idx - (long long)kx * N);
-    const C o = om[idx];
-    const double p = double(o.x) * double(o.x) + double(o.y) * double(o.y);
-    if (!isfinite(p)) bad = 1;
-    const double gz = double(z < Nh ? z : z - N);
-    const double K2 = double(kx) * double(kx) + gz * gz;
-    const double wt = (kx == 0 || kx == Nh - 1) ? 1.0 : 2.0;
-    if (K2 > 0.0) {
-      const double e = wt * p / K2;
-      csum_add(s[0], c[0], e);
-      csum_add(s[1], c[1], e / sqrt(K2));
-    } else {
-      csum_add(s[4], c[4], p);  // the (0,0) mode, removed from Z
+  for (int idx = blockIdx.x * NT + tid; idx < total; idx += gridDim.x * NT) {
+    const int kx = idx / (Nh + 1);
+    const int kz = idx - kx * (Nh + 1);
+    const C* __restrict__ col = om + (size_t)kx * N;
+    const C o = col[kz];
+    const double ox = widen(o.x), oy = widen(o.y);
+    double p = fma(ox, ox, oy * oy);
+    bad |= !finite_bits(p);
+    if (kz > 0 && kz < Nh) {
+      const C q = col[N - kz];
+      const double qx = widen(q.x), qy = widen(q.y);
+      const double p2 = fma(qx, qx, qy * qy);
+      bad |= !finite_bits(p2);
+      p += p2;
     }
-    csum_add(s[2], c[2], wt * p);
-    csum_add(s[3], c[3], wt * K2 * p);
+    const int k2 = kx * kx + kz * kz;
+    const double K2 = double(k2);
+    const double pw = (kx == 0 || kx == Nh - 1) ? p : p + p;
+    if (k2 > 0) {
+      const double r = int_rsqrt(K2, k2);
+      const double e = pw * r * r;
+      csum_add_pos(s[0], c[0], e);
+      csum_add_pos(s[1], c[1], e * r);
+    } else {
+      csum_add_pos(s[4], c[4], p);  // the (0,0) mode, removed from Z
+    }
+    csum_add_pos(s[2], c[2], pw);
+    csum_add_pos(s[3], c[3], K2 * pw);
   }
-  __shared__ double red[2 * 5 * (NT / 32)];
+  __shared__ double red[2 * 5 * NT];
   block_csum<NT, 5>(s, c, red, tid);
   if (bad) atomicOr(&a.sc->nonfinite, 1);
   if (tid == 0) {
@@ -1802,45 +1891,93 @@ __global__ void __launch_bounds__(NT) k_spectral(StepArgs a0) {
 // Energy spectrum of the compact vorticity band (turbo_simulator.py:2225-2357):
 // mode (kx, kz), K2 > 0, goes to bin floor((sqrt(K2)/k_nyq / r_max) nbins)
 // (clipped) with p = |om|^2 / K2 * scale2, doubled (and counted twice) for
-// kx > 0.  One block per bin: its threads walk the rows kz and only visit the
-// kx interval of that bin's annulus (float estimate plus a one-mode margin),
-// testing each mode with the reference's double-precision formula, so every
-// mode is counted exactly once and the sums are deterministic.
+// kx > 0.  K2 is an integer and the bin never falls as it grows, so bin b is
+// the K2 interval [edge[b], edge[b+1]), found once per bin with the reference's
+// double-precision formula (k_spectrum_edges); the binning itself then compares
+// integers.  One block per bin: its threads walk kz >= 0 and visit the kx of the
+// bin's annulus, taking kz and -kz together, so every mode is counted exactly
+// once and the sums are deterministic.  A bin narrower than a mode gives few
+// lanes one at a time: each warp lists its modes first and does the FP64 work
+// on full warps.  N=2048, 4096 bins: 1380 us with the formula per mode, 72 now.
+__device__ __forceinline__ int spectrum_bin(int k2, int nbins, double r_max, double k_nyq) {
+  const double r = sqrt((double)k2) / k_nyq;
+  const int bin = (int)floor((r / r_max) * (double)nbins);
+  return bin < 0 ? 0 : (bin >= nbins ? nbins - 1 : bin);
+}
+// edge[b], b = 0 .. nbins: the smallest K2 in 1 .. kmax2 + 1 whose bin is at
+// least b (kmax2 + 1 where there is none).
+template <int NT>
+__global__ void k_spectrum_edges(int* __restrict__ edge, int nbins, double r_max, double k_nyq, int kmax2) {
+  const int b = blockIdx.x * NT + threadIdx.x;
+  if (b > nbins) return;
+  int k = b == 0 ? 1 : kmax2 + 1;
+  if (b > 0 && b < nbins) {
+    const double t = (double)b * (r_max / (double)nbins) * k_nyq;
+    k = (int)fmin(fmax(t * t, 1.0), (double)kmax2 + 1.0);
+    while (k > 1 && spectrum_bin(k - 1, nbins, r_max, k_nyq) >= b) --k;
+    while (k <= kmax2 && spectrum_bin(k, nbins, r_max, k_nyq) < b) ++k;
+  }
+  edge[b] = k;
+}
 template <typename T, int NT>
-__global__ void __launch_bounds__(NT) k_spectrum(const cplx<T>* __restrict__ om, int N, int nbins, double r_max,
-                                                 double k_nyq, double scale2, double* __restrict__ esum,
-                                                 int* __restrict__ cnt) {
+__global__ void __launch_bounds__(NT) k_spectrum(const cplx<T>* __restrict__ om, int N, const int* __restrict__ edge,
+                                                 double scale2, double* __restrict__ esum, int* __restrict__ cnt) {
   const int b = blockIdx.x;
   const int Nh = N >> 1;
-  const float c = (float)(k_nyq * r_max / (double)nbins);  // annulus width in k
-  const float lo = b * c, hi = (b == nbins - 1) ? 3.0e38f : (b + 1) * c;
+  const int lo = edge[b], hi = edge[b + 1];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  __shared__ unsigned list[NT / 32][64];  // modes found by a warp and not yet summed: kx << 16 | kz
+  unsigned* buf = list[warp];
   double e = 0.0;
   long long n = 0;
-  for (int z = threadIdx.x; z < N; z += NT) {
-    const int kz = z < Nh ? z : z - N;
-    const float kz2 = (float)kz * (float)kz;
-    const float a = lo * lo - kz2;
-    int x0 = a > 0.f ? (int)floorf(sqrtf(a)) - 1 : 0;
-    const float h = hi * hi - kz2;
-    if (h < 0.f) continue;
-    int x1 = (hi > 1.0e37f) ? Nh - 1 : (int)ceilf(sqrtf(h)) + 1;
-    x0 = max(x0, 0);
-    x1 = min(x1, Nh - 1);
-    for (int kx = x0; kx <= x1; ++kx) {
-      const double k2 = (double)kx * (double)kx + (double)kz * (double)kz;
-      if (!(k2 > 0.0)) continue;
-      const double r = sqrt(k2) / k_nyq;
-      int bin = (int)floor((r / r_max) * (double)nbins);
-      bin = bin < 0 ? 0 : (bin >= nbins ? nbins - 1 : bin);
-      if (bin != b) continue;
-      const cplx<T> o = om[(size_t)kx * N + z];
-      double p = (((double)o.x * (double)o.x + (double)o.y * (double)o.y) / k2) * scale2;
-      const int wgt = kx > 0 ? 2 : 1;
-      if (wgt == 2) p *= 2.0;
-      e += p;
+  auto add = [&](unsigned mode) {
+    const int kx = (int)(mode >> 16), kz = (int)(mode & 0xffffu);
+    const cplx<T>* __restrict__ col = om + (size_t)kx * N;
+    const cplx<T> o = col[kz];
+    const double ox = widen(o.x), oy = widen(o.y);
+    double p = fma(ox, ox, oy * oy);
+    const int wgt = kx > 0 ? 2 : 1;
+    n += wgt;
+    if (kz > 0 && kz < Nh) {
+      const cplx<T> q = col[N - kz];
+      const double qx = widen(q.x), qy = widen(q.y);
+      p = fma(qx, qx, fma(qy, qy, p));
       n += wgt;
     }
+    const int k2 = kx * kx + kz * kz;
+    const double r = int_rsqrt((double)k2, k2);
+    p = p * (r * r) * scale2;
+    e += wgt == 2 ? p + p : p;
+  };
+  int held = 0;
+  for (int z0 = warp * 32; z0 <= Nh && z0 * z0 < hi; z0 += NT) {
+    // the kx of the annulus at kz, in integers (float estimates, corrected)
+    const int kz = z0 + lane;
+    int x0 = 0, x1 = -1;
+    if (kz <= Nh && kz * kz < hi) {
+      const int a = lo - kz * kz, h = hi - kz * kz;
+      x0 = max(a > 0 ? (int)sqrtf((float)a) - 1 : 0, 0);
+      while (x0 * x0 < a) ++x0;
+      x1 = (int)sqrtf((float)h) + 1;
+      while (x1 * x1 >= h) --x1;
+      x1 = min(x1, Nh - 1);
+    }
+    while (const unsigned have = __ballot_sync(0xffffffffu, x0 <= x1)) {
+      if (x0 <= x1) buf[held + __popc(have & ((1u << lane) - 1u))] = ((unsigned)x0 << 16) | (unsigned)kz;
+      ++x0;
+      held += __popc(have);
+      __syncwarp();
+      if (held >= 32) {
+        const unsigned mode = buf[lane], rest = buf[32 + lane];
+        __syncwarp();
+        held -= 32;
+        if (lane < held) buf[lane] = rest;
+        __syncwarp();
+        add(mode);
+      }
+    }
   }
+  if (lane < held) add(buf[lane]);
   __shared__ double red[2 * (NT / 32)];
   double v[2] = {e, (double)n};
   block_sum<NT, 2>(v, red, threadIdx.x);

@@ -7,6 +7,7 @@
 // twiddle tables.  pal_create times every candidate on the handle's own state
 // and keeps the fastest (pal_autotune in pal_api.cu).
 #pragma once
+#include <algorithm>
 #include <cstdlib>
 
 #include "pal_adjoint.cuh"
@@ -71,7 +72,7 @@ struct KernelSet {
   void (*spectral)(const StepArgs&, cudaStream_t, int blocks);
   void (*transpose)(const void* in, void* out, int rows, int cols, int batch, cudaStream_t);
   void (*spectrum)(const void* om, int N, int nbins, double r_max, double k_nyq, double scale2, double* esum, int* cnt,
-                   cudaStream_t);
+                   int* edge, cudaStream_t);  // edge: nbins + 1 ints of scratch
   // display: |u| into plane 2 of `phys`, and min/max -> 8-bit pixels of one plane
   void (*speed)(void* phys, long long plane, cudaStream_t);
   void (*pixels)(const void* plane, long long n, double* part, unsigned int* counter, double* mm, unsigned char* pix,
@@ -118,6 +119,16 @@ inline int wave_blocks(K kernel, int nt, size_t smem) {
   return sms * per_sm;
 }
 
+// Blocks per member of a pass that loops over `tiles` tiles: at most one wave
+// over all members, and tile counts that differ by at most one between blocks
+// (0: the wave is not known).
+inline int phys_blocks(int tiles, int wave, int members) {
+  const int most = wave / members > 0 ? wave / members : tiles;
+  if (most >= tiles) return tiles;
+  const int rounds = (tiles + most - 1) / most;
+  return (tiles + rounds - 1) / rounds;
+}
+
 // Column-pass flags of LS-IMEX-RK3 stage s (0..2) on butterfly-major om /
 // fnm1: the first stage reads no fnm1, the first two hand the next stage its
 // combined q in om (k_col F_Q_OUT / F_Q_IN), the last stores om and fn.
@@ -129,7 +140,7 @@ __host__ __device__ inline void rk3_stage_flags(StepArgs& a, int s, const double
 
 template <typename T, class PL, int V, int NT, int PF = 0>
 struct RowOf {
-  static constexpr size_t smem = size_t(PL::PADM) * V * sizeof(cplx<T>);
+  static constexpr size_t smem = std::max(size_t(PL::PADM) * V * sizeof(cplx<T>), size_t(2) * NT * sizeof(double));
   static_assert(smem <= kSmemLimit, "row tile does not fit in shared memory");
   static_assert(PL::M % V == 0, "row tile must divide M");
   static inline int ahead = 0;
@@ -146,7 +157,9 @@ struct RowOf {
       if (e != cudaSuccess) return e;
     }
     if (PF & 1) ahead = ((PF & 32) ? 2 : 1) * wave_blocks(k_row<T, PL, V, NT, PF>, NT, smem);
-    return cudaFuncSetAttribute(k_phys<T, PL, V, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = cudaFuncSetAttribute(k_phys<T, PL, V, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) phys_wave = wave_blocks(k_phys<T, PL, V, NT>, NT, smem);
+    return e;
   }
   static void row(const StepArgs& a, cudaStream_t s) {
     StepArgs b = a;
@@ -155,8 +168,12 @@ struct RowOf {
     k_row<T, PL, V, NT, PF><<<dim3(PL::M / V, a.members > 1 ? a.members : 1), NT, smem, s>>>(
         b, ((PF & 12) != 0 && a.tmaps) ? *a.tmaps : none);
   }
+  // k_phys: one wave of blocks shared by the members, each looping over its
+  // member's tiles
+  static inline int phys_wave = 0;
   static void phys(const StepArgs& a, cudaStream_t s) {
-    k_phys<T, PL, V, NT><<<dim3(PL::M / V, a.members > 1 ? a.members : 1), NT, smem, s>>>(a);
+    const int m = a.members > 1 ? a.members : 1;
+    k_phys<T, PL, V, NT><<<dim3(phys_blocks(PL::M / V, phys_wave, m), m), NT, smem, s>>>(a);
   }
   static int blocks_per_sm() {
     int n = 0;
@@ -294,11 +311,17 @@ struct RowFxOf {
   static_assert(smem <= kSmemLimit && PL::M % V == 0 && NT % 32 == 0, "row tile, whole warps");
   static cudaError_t configure() {
     cudaError_t e = set_tile_smem(k_row_fx<FP, V, NT, MINB>, smem);
-    return e == cudaSuccess ? set_tile_smem(k_phys_fx<FP, V, NT>, smem) : e;
+    if (e == cudaSuccess) e = set_tile_smem(k_phys_fx<FP, V, NT>, smem);
+    if (e == cudaSuccess) phys_wave = wave_blocks(k_phys_fx<FP, V, NT>, NT, smem);
+    return e;
   }
+  static inline int phys_wave = 0;
   static dim3 grid(const StepArgs& a) { return dim3(PL::M / V, a.members > 1 ? a.members : 1); }
   static void row(const StepArgs& a, cudaStream_t s) { k_row_fx<FP, V, NT, MINB><<<grid(a), NT, smem, s>>>(a); }
-  static void phys(const StepArgs& a, cudaStream_t s) { k_phys_fx<FP, V, NT><<<grid(a), NT, smem, s>>>(a); }
+  static void phys(const StepArgs& a, cudaStream_t s) {
+    const dim3 g = grid(a);
+    k_phys_fx<FP, V, NT><<<dim3(phys_blocks(g.x, phys_wave, g.y), g.y), NT, smem, s>>>(a);
+  }
   static int blocks_per_sm() {
     int n = 0;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_row_fx<FP, V, NT, MINB>, NT, smem) == cudaSuccess ? n : -1;
@@ -397,9 +420,10 @@ void launch_transpose(const void* in, void* out, int rows, int cols, int batch, 
 
 template <typename T>
 void launch_spectrum(const void* om, int N, int nbins, double r_max, double k_nyq, double scale2, double* esum,
-                     int* cnt, cudaStream_t s) {
-  k_spectrum<T, 256><<<nbins, 256, 0, s>>>(static_cast<const cplx<T>*>(om), N, nbins, r_max, k_nyq, scale2, esum,
-                                             cnt);
+                     int* cnt, int* edge, cudaStream_t s) {
+  const int nh = N / 2, kmax2 = (nh - 1) * (nh - 1) + nh * nh;
+  k_spectrum_edges<32><<<nbins / 32 + 1, 32, 0, s>>>(edge, nbins, r_max, k_nyq, kmax2);
+  k_spectrum<T, 128><<<nbins, 128, 0, s>>>(static_cast<const cplx<T>*>(om), N, edge, scale2, esum, cnt);
 }
 
 template <typename T>

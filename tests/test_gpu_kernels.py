@@ -157,3 +157,62 @@ def test_fixed_point_non_finite_fields(N, bad):
     F.step("LS_IMEX_RK3", 2)
     assert not F.om2().any() and not F.ur(0).any()
     F.close()
+
+
+@pytest.mark.parametrize("nbins, r_max, k_nyq", [(1, 1.0, 16.0), (7, 0.3, 10.0), (32, 2.0**0.5, 16.0),
+                                                 (1000, 2.0**0.5, 192.0), (513, 5.0, 3.0), (64, 1e-3, 1e-3)])
+@pytest.mark.parametrize("N, prec", [(32, "fp32"), (384, "fp64")])
+def test_energy_spectrum_bins(N, prec, nbins, r_max, k_nyq):
+    """Bins as intervals of the integer K2 against the per-mode formula, at
+    widths from many modes a bin to many bins a mode."""
+    from palinstrophy_gb300.turbo_simulator import Field
+
+    om = _spectrum(N, "k-1").astype(np.complex64 if prec == "fp32" else np.complex128)
+    F = Field(N, prec, 1e3, 0.3)
+    F.set_state(om)
+    e, c = F.energy_spectrum(nbins, r_max, k_nyq)
+    F.close()
+    nh = N // 2
+    kx = np.arange(nh, dtype=np.float64)[None, :]
+    kz = np.where(np.arange(N) < nh, np.arange(N), np.arange(N) - N).astype(np.float64)[:, None]
+    k2 = kx * kx + kz * kz
+    with np.errstate(over="ignore"):
+        b = np.clip(np.floor(np.sqrt(k2) / k_nyq / r_max * nbins), 0, nbins - 1).astype(np.int64)
+    w = np.where(kx > 0, 2, 1) * (k2 > 0)
+    o = om.astype(np.complex128)
+    p = w * (o.real**2 + o.imag**2) / np.where(k2 > 0, k2, 1.0) * (1.5 * N) ** 4
+    assert np.array_equal(c, np.bincount(b.ravel(), w.ravel(), nbins).astype(np.int64))
+    ref = np.bincount(b.ravel(), p.ravel(), nbins)
+    # positive terms: at most N^2/2 additions of one rounding each, on both sides
+    assert np.all(np.abs(e - ref) <= N * N * np.finfo(np.float64).eps * ref)
+
+
+@pytest.mark.parametrize("prec", ["fp32", "fp64"])
+@pytest.mark.parametrize("N", [32, 96 * 4, 1024])
+def test_spectral_sums(N, prec):
+    """E, L, Z, P of k_spectral against exactly rounded sums (math.fsum): the
+    terms carry a few FP64 roundings each, the sums none."""
+    import math
+
+    from palinstrophy_gb300.turbo_simulator import Field
+
+    om = _spectrum(N, "k-1").astype(np.complex64 if prec == "fp32" else np.complex128)
+    om[0, 0] = 0.25
+    F = Field(N, prec, 1e3, 0.3)
+    F.set_state(om)
+    F.set_scalars(dt=1e-3)
+    d = F.diagnostics()
+    F.close()
+    nh = N // 2
+    kx = np.arange(nh, dtype=np.float64)[None, :]
+    kz = np.where(np.arange(N) < nh, np.arange(N), np.arange(N) - N).astype(np.float64)[:, None]
+    k2 = kx * kx + kz * kz
+    w = np.where((kx == 0) | (kx == nh - 1), 1.0, 2.0) * np.ones_like(k2)
+    o = om.astype(np.complex128)
+    p = w * (o.real**2 + o.imag**2)
+    m = k2 > 0
+    E = math.fsum((p[m] / k2[m]).ravel())
+    S = math.fsum((p[m] / k2[m] / np.sqrt(k2[m])).ravel())
+    for key, ref in (("E", E), ("L", 2.0 * math.pi * S / E), ("Z", math.fsum(p.ravel()) - p[0, 0]),
+                     ("P", math.fsum((k2 * p).ravel()))):
+        assert abs(d[key] - ref) <= 16 * np.finfo(np.float64).eps * ref, key
