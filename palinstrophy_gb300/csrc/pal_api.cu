@@ -46,6 +46,7 @@ struct pal_handle {
   const ColKernels* ck = nullptr;  // selected column-pass candidate
   int row_idx = 0, col_idx = 0;
   cudaStream_t stream = nullptr;
+  void* arena = nullptr;  // one allocation holding w0 .. part below
   void *w0 = nullptr, *w1 = nullptr, *om = nullptr, *fnm1 = nullptr;
   void *om_p = nullptr, *fm_p = nullptr;  // om / fnm1 in butterfly-major order, used inside pal_step
   pal::TmaMaps tmaps{};                   // w0 / w1 descriptors when the row candidate moves rows by TMA
@@ -285,6 +286,10 @@ int select_variant(pal_handle* h, int row, int col) {
   h->step_graphs.clear();
   h->rk = &h->ks->rows[row];
   h->ck = &h->ks->cols[col];
+  // kernel attributes of the two candidates only: a handle of a tuned size sets
+  // a dozen instead of every candidate's
+  PAL_CK(h, h->rk->configure());
+  PAL_CK(h, h->ck->configure());
   if (h->rk->tma && !pal::encode_row_maps(&h->tmaps, h->w0, h->w1, h->N, h->rk->V, 1))
     return fail(h, PAL_ERR_CUDA, "TMA descriptor of the work planes could not be encoded");
   if (h->ck->tma && !pal::encode_col_maps(&h->cmaps, h->w0, h->w1, h->N, h->ck->rp, 1))
@@ -493,15 +498,8 @@ int pal_create(int N, int precision, double Re, double cfl, pal_handle** out) {
   };
   cudaError_t e = cudaSuccess;
   size_t tw_max = 0;
-  for (int r = 0; r < ks->n_rows && e == cudaSuccess; ++r) {
-    e = ks->rows[r].configure();
-    tw_max = std::max(tw_max, (size_t)ks->rows[r].tw_elems);
-  }
-  for (int c = 0; c < ks->n_cols && e == cudaSuccess; ++c) {
-    e = ks->cols[c].configure();
-    tw_max = std::max(tw_max, (size_t)ks->cols[c].tw_elems);
-  }
-  if (e != cudaSuccess) return bail(cuda_fail(nullptr, e, "kernel configure"));
+  for (int r = 0; r < ks->n_rows; ++r) tw_max = std::max(tw_max, (size_t)ks->rows[r].tw_elems);
+  for (int c = 0; c < ks->n_cols; ++c) tw_max = std::max(tw_max, (size_t)ks->cols[c].tw_elems);
   e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) return bail(cuda_fail(nullptr, e, "cudaStreamCreate"));
   const size_t plane_w = (size_t)h->Nh * h->M * h->esz;
@@ -512,20 +510,26 @@ int pal_create(int N, int precision, double Re, double cfl, pal_handle** out) {
   // two blocks per SM: a block's FP64 reduction tree costs as much as ten modes per thread
   h->spectral_blocks = std::max(1, std::min(2 * sms, (int)(((size_t)N * h->Nh + 255) / 256)));
   const size_t part_n = (size_t)std::max(h->M, std::max(1024, h->spectral_blocks)) * 5;
-  void** bufs[] = {&h->w0, &h->w1, &h->om, &h->fnm1, &h->stage, &h->tw_row, &h->tw_col, &h->om_p};
+  // the state in one allocation (an allocation and its release cost 10 to 30 us
+  // each, which a short-lived handle notices), every array on a 256-byte boundary
+  void** bufs[] = {&h->w0, &h->w1, &h->om, &h->fnm1, &h->stage, &h->tw_row, &h->tw_col, &h->om_p,
+                   reinterpret_cast<void**>(&h->sc), reinterpret_cast<void**>(&h->part)};
   const size_t sizes[] = {plane_w + pal::kPlaneSlack, plane_w + pal::kPlaneSlack, plane_om, plane_om, 2 * plane_om,
-                          tw_max * h->esz, tw_max * h->esz, 2 * plane_w};
-  for (int i = 0; i < 8; ++i) {
-    e = cudaMalloc(bufs[i], sizes[i]);
-    if (e != cudaSuccess) return bail(cuda_fail(nullptr, e, "cudaMalloc state"));
-    e = cudaMemsetAsync(*bufs[i], 0, sizes[i], h->stream);
-    if (e != cudaSuccess) return bail(cuda_fail(nullptr, e, "cudaMemset state"));
+                          tw_max * h->esz, tw_max * h->esz, 2 * plane_w, sizeof(DevScalars), part_n * sizeof(double)};
+  constexpr int n_bufs = sizeof(sizes) / sizeof(sizes[0]);
+  auto padded = [](size_t n) { return (n + 255) & ~(size_t)255; };
+  size_t total = 0;
+  for (size_t n : sizes) total += padded(n);
+  e = cudaMalloc(&h->arena, total);
+  if (e != cudaSuccess) return bail(cuda_fail(nullptr, e, "cudaMalloc state"));
+  e = cudaMemsetAsync(h->arena, 0, total, h->stream);
+  if (e != cudaSuccess) return bail(cuda_fail(nullptr, e, "cudaMemset state"));
+  char* at = static_cast<char*>(h->arena);
+  for (int i = 0; i < n_bufs; ++i) {
+    *bufs[i] = at;
+    at += padded(sizes[i]);
   }
   h->fm_p = static_cast<char*>(h->om_p) + plane_w;
-  e = cudaMalloc(&h->sc, sizeof(DevScalars));
-  if (e != cudaSuccess) return bail(cuda_fail(nullptr, e, "cudaMalloc scalars"));
-  e = cudaMalloc(&h->part, part_n * sizeof(double));
-  if (e != cudaSuccess) return bail(cuda_fail(nullptr, e, "cudaMalloc partials"));
   e = cudaMallocHost(&h->sc_host, sizeof(DevScalars));
   if (e != cudaSuccess) return bail(cuda_fail(nullptr, e, "cudaMallocHost"));
   std::memset(h->sc_host, 0, sizeof(DevScalars));
@@ -549,9 +553,7 @@ int pal_destroy(pal_handle* h) {
   if (h->stream) cudaStreamSynchronize(h->stream);
   for (auto& kv : h->step_graphs) cudaGraphExecDestroy(kv.second);
   h->step_graphs.clear();
-  void* bufs[] = {h->w0,     h->w1,   h->om,   h->fnm1, h->stage, h->tw_row,   h->tw_col,
-                  h->phys,   h->sc,   h->part, h->vis_w, h->vis_phys, h->om_p,
-                  h->spec};
+  void* bufs[] = {h->arena, h->phys, h->vis_w, h->vis_phys, h->spec};
   for (void* b : bufs)
     if (b) cudaFree(b);
   if (h->spec_host) cudaFreeHost(h->spec_host);
@@ -907,136 +909,154 @@ int pal_adjoint_palinstrophy(pal_handle* h, int nsteps, int ckpt_every, double* 
   if (h->state != ST_U) return fail(h, PAL_ERR_STATE, "adjoint needs the physical velocity");
   if (adj->configure() != cudaSuccess) return fail(h, PAL_ERR_CUDA, "adjoint configure");
   const size_t plane_om = (size_t)h->Nh * h->N * h->esz, plane_w = (size_t)h->Nh * h->M * h->esz;
-  const int n_ck = (nsteps + ckpt_every - 1) / ckpt_every;
-  const int stages_max = 3 * ckpt_every;
-  // one allocation: checkpoints (om, fnm1) | final state | stage inputs | lam_om, lam_f | Y planes | tables | loss
+  // Segments of `seg` steps: their stages' velocity planes (two of plane_w each)
+  // are kept while the segment runs backward.  ckpt_every steps, or a third of
+  // that where the planes would take more than 1 GiB (they are three times the
+  // stage's om; a shorter segment costs checkpoints, not recomputation).
+  const size_t per_step = 3 * 2 * plane_w;
+  const int seg = std::min(nsteps, (size_t)ckpt_every * per_step <= ((size_t)1 << 30) ? ckpt_every : (ckpt_every + 2) / 3);
+  const int n_ck = (nsteps + seg - 1) / seg;
+  // one allocation: checkpoints (om, fnm1, butterfly-major) of all segments but the last |
+  // velocity planes of a segment's stages and of its end | om, fnm1 of the segment, lam_om, lam_f |
+  // twiddle tables | loss
   const size_t tw_bytes = (size_t)(adj->tw_row_elems + adj->tw_col_elems) * h->esz;
-  const int seed_blocks = 256;
-  const size_t bytes = 2 * plane_om * (size_t)n_ck + 2 * plane_om + plane_om * (size_t)stages_max + 2 * plane_om +
-                       2 * plane_w + tw_bytes + seed_blocks * sizeof(double) + 1024;
+  const size_t bytes = 2 * plane_w * (size_t)(n_ck - 1) + per_step * (size_t)seg + 6 * plane_w + tw_bytes +
+                       h->Nh * sizeof(double) + 1024;
   char* buf = nullptr;
   PAL_CK(h, cudaMallocAsync(reinterpret_cast<void**>(&buf), bytes, h->stream));
   char* ck = buf;
-  char* fin = ck + 2 * plane_om * (size_t)n_ck;
-  char* st = fin + 2 * plane_om;
-  char* lom = st + plane_om * (size_t)stages_max;
-  char* lf = lom + plane_om;
-  char* y0 = lf + plane_om;
-  char* y1 = y0 + plane_w;
-  char* tw_r = y1 + plane_w;
+  char* st = ck + 2 * plane_w * (size_t)(n_ck - 1);
+  char* bo = st + per_step * (size_t)seg + 2 * plane_w;
+  char* bf = bo + plane_w;
+  char* lom = bf + plane_w;
+  char* lf = lom + plane_w;
+  char* tw_r = lf + plane_w;
   char* tw_c = tw_r + (size_t)adj->tw_row_elems * h->esz;
   double* loss_part = reinterpret_cast<double*>(((uintptr_t)(tw_c + (size_t)adj->tw_col_elems * h->esz) + 255) & ~(uintptr_t)255);
   adj->tw_row(tw_r, h->stream);
   adj->tw_col(tw_c, h->stream);
+  auto seg_len = [&](int k) { return std::min(seg, nsteps - k * seg); };
+  // arguments of stage q of a segment: its velocity planes as y0, y1
+  auto stage_args = [&](int q, void* om, void* fm, void* tw) {
+    StepArgs a = base_args(h);
+    a.om_p = om;
+    a.fm_p = fm;
+    a.y0 = st + 2 * plane_w * (size_t)q;
+    a.y1 = st + 2 * plane_w * (size_t)q + plane_w;
+    a.tw = tw;
+    a.scheme = 1;
+    a.alpha = kRkAlpha[q % 3];
+    a.beta = kRkBeta[q % 3];
+    return a;
+  };
+  // stages 0 .. n - 1 of a segment forward from bo / bf, their velocity planes kept (stage 0's are
+  // there already)
+  auto keep_stages = [&](int n, bool advance) -> int {
+    for (int q = 0; q < n; ++q) {
+      adj->fwd_row(stage_args(q, bo, bf, tw_r), h->stream);
+      StepArgs c = stage_args(q, bo, bf, tw_c);
+      const StepArgs next = stage_args(q + 1, bo, bf, tw_c);
+      c.y0 = next.y0;
+      c.y1 = next.y1;
+      if (advance && q % 3 == 2) c.flags = pal::F_ADVANCE;
+      adj->fwd_col(c, h->stream);
+    }
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? PAL_OK : cuda_fail(h, e, "adjoint forward stage");
+  };
+  auto backward = [&](int ns) -> int {
+    for (int q = 3 * ns; q >= 0; --q) {
+      // the end of stage q and the start of stage q - 1
+      StepArgs a = stage_args(q > 0 ? q - 1 : 0, lom, lf, tw_c);
+      a.flags = (q < 3 * ns ? pal::F_ADJ_OUT : 0) | (q > 0 ? pal::F_ADJ_IN : 0);
+      adj->col(a, h->stream);
+      if (q > 0) adj->row(stage_args(q - 1, lom, lf, tw_r), h->stream);
+    }
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? PAL_OK : cuda_fail(h, e, "adjoint stage");
+  };
   int rc = PAL_OK;
-  auto seg_len = [&](int seg) { return std::min(ckpt_every, nsteps - seg * ckpt_every); };
-  // Segments are launch sequences with fixed buffers; full-length segments are
-  // captured once as CUDA graphs (forward, and recompute + adjoint sweep) and
-  // replayed, the checkpoint copies staying outside the graphs.
-  auto forward_body = [&](int ns) -> int {
-    int r = PAL_OK;
-    for (int j = 0; j < ns && r == PAL_OK; ++j) r = one_step(h, PAL_LS_IMEX_RK3, false, true);
-    return r;
-  };
-  auto backward_body = [&](int ns) -> int {
-    h->state = ST_VEL_PENDING;
-    h->vel_uploaded = false;
-    int r = resolve_velocity(h);
-    for (int j = 0; j < ns && r == PAL_OK; ++j) {
-      for (int s = 0; s < 3 && r == PAL_OK; ++s) {
-        cudaMemcpyAsync(st + plane_om * (size_t)(3 * j + s), h->om, plane_om, cudaMemcpyDeviceToDevice, h->stream);
-        if ((r = launch_row(h, 0))) break;
-        r = launch_col(h, 1, s, 0);
-      }
-    }
-    for (int q = 3 * ns - 1; q >= 0 && r == PAL_OK; --q) {
-      const int s = q % 3;
-      StepArgs a = base_args(h);
-      a.om = lom;
-      a.fnm1 = lf;
-      a.alpha = kRkAlpha[s];
-      a.beta = kRkBeta[s];
-      a.tw = tw_c;
-      adj->col_in(a, h->stream);
-      StepArgs b = base_args(h);
-      b.om = st + plane_om * (size_t)q;
-      b.w0 = y0;
-      b.w1 = y1;
-      b.tw = tw_c;
-      b.src = nullptr;
-      adj->col_vel(b, h->stream);
-      a.y0 = y0;
-      a.y1 = y1;
-      a.tw = tw_r;
-      adj->row(a, h->stream);
-      a.tw = tw_c;
-      adj->col_out(a, h->stream);
-      cudaError_t e = cudaGetLastError();
-      if (e != cudaSuccess) r = cuda_fail(h, e, "adjoint stage");
-    }
-    return r;
-  };
-  auto capture = [&](auto&& body, int ns, cudaGraphExec_t* exec) -> int {
+  auto capture = [&](auto&& body, cudaGraphExec_t* exec) -> int {
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return cuda_fail(h, e, "begin capture");
-    const int r = body(ns);
+    const int r = body();
     e = cudaStreamEndCapture(h->stream, &g);
-    if (r) return r;
+    if (r) {
+      if (g) cudaGraphDestroy(g);
+      return r;
+    }
     if (e != cudaSuccess) return cuda_fail(h, e, "end capture");
     e = cudaGraphInstantiate(exec, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) return cuda_fail(h, e, "graph instantiate");
     return PAL_OK;
   };
-  const bool use_graphs = !(std::getenv("PAL_ADJOINT_GRAPHS") && std::getenv("PAL_ADJOINT_GRAPHS")[0] == '0');
+  // Full segments before the last repeat one launch sequence with fixed buffers:
+  // captured once each as CUDA graphs (forward; kept stages and backward sweep)
+  // where there are enough of them to pay for the capture.
+  const char* genv = std::getenv("PAL_ADJOINT_GRAPHS");
+  const bool use_graphs = !(genv && genv[0] == '0') && n_ck - 1 >= 3;
   cudaGraphExec_t g_fwd = nullptr, g_bwd = nullptr;
-  // forward sweep with checkpoints (fixed dt: no NEXTDT)
-  for (int seg = 0; seg < n_ck && rc == PAL_OK; ++seg) {
-    cudaMemcpyAsync(ck + 2 * plane_om * seg, h->om, plane_om, cudaMemcpyDeviceToDevice, h->stream);
-    cudaMemcpyAsync(ck + 2 * plane_om * seg + plane_om, h->fnm1, plane_om, cudaMemcpyDeviceToDevice, h->stream);
-    const int ns = seg_len(seg);
-    if (use_graphs && ns == ckpt_every) {
-      if (!g_fwd) rc = capture(forward_body, ns, &g_fwd);
-      if (rc == PAL_OK && cudaGraphLaunch(g_fwd, h->stream) != cudaSuccess) rc = fail(h, PAL_ERR_CUDA, "graph launch");
-    } else {
-      rc = forward_body(ns);
-    }
+  auto vel_first = [&]() { adj->vel(stage_args(0, bo, bf, tw_c), h->stream); };
+  // a segment that is run again later: its end's velocity becomes the next one's first
+  auto forward_body = [&]() -> int {
+    const int r = keep_stages(3 * seg, true);
+    cudaMemcpyAsync(st, st + per_step * (size_t)seg, 2 * plane_w, cudaMemcpyDeviceToDevice, h->stream);
+    return r;
+  };
+  auto backward_body = [&]() -> int {
+    vel_first();
+    const int r = keep_stages(3 * seg - 1, false);  // the last stage's own end is not needed
+    return r != PAL_OK ? r : backward(seg);
+  };
+  auto run = [&](auto&& body, cudaGraphExec_t* exec) -> int {
+    if (!use_graphs) return body();
+    if (!*exec)
+      if (int r = capture(body, exec)) return r;
+    return cudaGraphLaunch(*exec, h->stream) == cudaSuccess ? PAL_OK : fail(h, PAL_ERR_CUDA, "graph launch");
+  };
+  // forward sweep with checkpoints (fixed dt: no NEXTDT); the last segment keeps its stages
+  StepArgs state = base_args(h);
+  state.om_p = bo;
+  state.fm_p = bf;
+  adj->to_perm(state, h->stream);
+  vel_first();
+  for (int k = 0; k + 1 < n_ck && rc == PAL_OK; ++k) {
+    cudaMemcpyAsync(ck + 2 * plane_w * (size_t)k, bo, 2 * plane_w, cudaMemcpyDeviceToDevice, h->stream);
+    rc = run(forward_body, &g_fwd);
   }
+  if (rc == PAL_OK) rc = keep_stages(3 * seg_len(n_ck - 1), true);
   if (rc == PAL_OK) {
-    cudaMemcpyAsync(fin, h->om, plane_om, cudaMemcpyDeviceToDevice, h->stream);
-    cudaMemcpyAsync(fin + plane_om, h->fnm1, plane_om, cudaMemcpyDeviceToDevice, h->stream);
-    adj->seed(h->om, lom, lf, h->N, loss_part, seed_blocks, h->stream);
+    adj->from_perm(state, h->stream);
+    adj->seed(h->om, lom, lf, loss_part, h->stream);
+    rc = backward(seg_len(n_ck - 1));
   }
-  // backward sweep: per segment, recompute and store the stage inputs, then run
-  // the adjoint stages in reverse
-  for (int seg = n_ck - 1; seg >= 0 && rc == PAL_OK; --seg) {
-    cudaMemcpyAsync(h->om, ck + 2 * plane_om * seg, plane_om, cudaMemcpyDeviceToDevice, h->stream);
-    cudaMemcpyAsync(h->fnm1, ck + 2 * plane_om * seg + plane_om, plane_om, cudaMemcpyDeviceToDevice, h->stream);
-    const int ns = seg_len(seg);
-    if (use_graphs && ns == ckpt_every) {
-      if (!g_bwd) rc = capture(backward_body, ns, &g_bwd);
-      if (rc == PAL_OK && cudaGraphLaunch(g_bwd, h->stream) != cudaSuccess) rc = fail(h, PAL_ERR_CUDA, "graph launch");
-    } else {
-      rc = backward_body(ns);
-    }
+  // backward sweep: each segment's stages again, then their adjoints in reverse
+  for (int k = n_ck - 2; k >= 0 && rc == PAL_OK; --k) {
+    cudaMemcpyAsync(bo, ck + 2 * plane_w * (size_t)k, 2 * plane_w, cudaMemcpyDeviceToDevice, h->stream);
+    rc = run(backward_body, &g_bwd);
   }
   if (g_fwd) cudaGraphExecDestroy(g_fwd);
   if (g_bwd) cudaGraphExecDestroy(g_bwd);
-  // leave the handle at the final forward state
-  cudaMemcpyAsync(h->om, fin, plane_om, cudaMemcpyDeviceToDevice, h->stream);
-  cudaMemcpyAsync(h->fnm1, fin + plane_om, plane_om, cudaMemcpyDeviceToDevice, h->stream);
+  // the handle is at the final forward state; its work planes served the sweeps
   h->state = ST_VEL_PENDING;
   h->vel_uploaded = false;
   if (rc == PAL_OK) rc = resolve_velocity(h);
   if (rc == PAL_OK && grad_host) {
-    h->ks->transpose(lom, h->stage, h->Nh, h->N, 1, h->stream);
+    // lam_om back to natural columns (in bo), then to the reference layout
+    StepArgs p = base_args(h);
+    p.om = bo;
+    p.om_p = lom;
+    p.flags = pal::F_NO_FM_IN;
+    adj->from_perm(p, h->stream);
+    h->ks->transpose(bo, h->stage, h->Nh, h->N, 1, h->stream);
     cudaError_t e = cudaMemcpyAsync(grad_host, h->stage, plane_om, cudaMemcpyDeviceToHost, h->stream);
     if (e != cudaSuccess) rc = cuda_fail(h, e, "gradient download");
   }
-  std::vector<double> lp(seed_blocks, 0.0);
+  std::vector<double> lp(h->Nh, 0.0);
   if (rc == PAL_OK && loss) {
-    cudaError_t e = cudaMemcpyAsync(lp.data(), loss_part, seed_blocks * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
+    cudaError_t e = cudaMemcpyAsync(lp.data(), loss_part, h->Nh * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
     if (e != cudaSuccess) rc = cuda_fail(h, e, "loss download");
   }
   cudaFreeAsync(buf, h->stream);

@@ -210,6 +210,15 @@ __device__ __forceinline__ double fx_small(int i) {
 __device__ __forceinline__ bool fx_normal(int E) { return E >= -1020 && E <= 950; }
 __device__ __noinline__ static double fx_scalbn(long long q, int E) { return scalbn(fx_to_double(q, 0), E); }
 
+// 1 / d by two steps of Newton's iteration from the hardware's reciprocal
+// estimate (about 20 bits: each step doubles them).  d is finite and at least 1.
+__device__ __forceinline__ double newton_rcp(double d) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+  r = fma(r, fma(-d, r, 1.0), r);
+  return fma(r, fma(-d, r, 1.0), r);
+}
+
 // cos and sin of pi/4 * r / M (0 <= r <= M) as 63-bit fractions, by their Taylor
 // series in integers (eleven terms: below 2^-63 for arguments up to pi/4).
 __device__ __forceinline__ unsigned long long fx_mul63(unsigned long long a, unsigned long long b) {

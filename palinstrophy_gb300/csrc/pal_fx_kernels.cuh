@@ -242,24 +242,43 @@ __device__ __forceinline__ void fx_rows_inverse(const void* p0, const void* p1, 
   fx_dif<PL, V, NT, +1, 1, PL::NP, 0>(sm, tw, tid, ws, sc);
 }
 
+// Unpack P = FFT(a + i b) (natural order, largest word in bits[NP]) into A =
+// F(a), B = F(b) for kx < N/2.
+template <class PL, int V, int NT>
+__device__ __forceinline__ void fx_rows_unpack(void* p0, void* p1, const fxc* sm, int z0, int tid, const FxWords* ws,
+                                               const FxScale& sc) {
+  constexpr int M = PL::M, Nh = M / 3, NP = PL::NP;
+  double2* __restrict__ w0 = static_cast<double2*>(p0);
+  double2* __restrict__ w1 = static_cast<double2*>(p1);
+  const int s = min(fx_shift_exact(ws->bits[NP], 62), 0);  // room for the sums
+  const FxScale out{sc.E - s - 1, sc.bad};
+  for (int w = tid; w < V * Nh; w += NT) {
+    const int v = w % V;
+    const int k = w / V;
+    fxc p[2] = {sm[PL::phys(k) * V + v], sm[PL::phys(k == 0 ? 0 : M - k) * V + v]};
+    fx_rescale<2>(p, s);
+    const size_t at = (size_t)k * M + z0 + v;
+    w0[at] = make_double2(fx_value(p[0].x + p[1].x, out), fx_value(p[0].y - p[1].y, out));
+    w1[at] = make_double2(fx_value(p[0].y + p[1].y, out), fx_value(p[1].x - p[0].x, out));
+  }
+}
+
 // k_row in fixed point: U-state rows -> products -> P-state rows, optional CFL
 // statistics.  Bound by the integer pipes (ncu: ALU 55 % of its rate, the
 // widening multiply-adds most of the rest) and, with one or two tiles per SM, by
 // the latency between its passes.  N=4096 1190 us (FP64 transforms: 6120, the
 // FP64 pipe 83 % busy), N=1024 70 us (352).
-template <class PL, int V, int NT, int MINB>
-__global__ void __launch_bounds__(NT, MINB) k_row_fx(StepArgs a0) {
-  const Blk bk = hw_blk();
-  const StepArgs a = member_args(a0, sizeof(double2), bk.y);
+template <class PL, int V, int NT>
+__device__ __forceinline__ void row_fx_body(const StepArgs& a, const void* u0, const void* u1, const Blk bk) {
   extern __shared__ __align__(128) unsigned char smraw[];
   __shared__ FxWords ws;
   fxc* sm = reinterpret_cast<fxc*>(smraw);
-  constexpr int M = PL::M, Nh = M / 3, NP = PL::NP;
+  constexpr int M = PL::M, NP = PL::NP;
   const int tid = threadIdx.x;
   const int z0 = bk.x * V;
   const int4* __restrict__ tw = static_cast<const int4*>(a.tw);
   FxScale sc;
-  fx_rows_inverse<PL, V, NT>(a.w0, a.w1, sm, tw, z0, tid, &ws, sc);
+  fx_rows_inverse<PL, V, NT>(u0, u1, sm, tw, z0, tid, &ws, sc);
 
   // products u^2 - v^2, u v of the inverse transform's points, divided by 2^64,
   // and the first forward pass on them: u, v are brought below 2^KU
@@ -307,21 +326,14 @@ __global__ void __launch_bounds__(NT, MINB) k_row_fx(StepArgs a0) {
   }
   fx_dit<PL, V, NT, -1, NP - 2, 0, NP>(sm, tw, tid, &ws, sc);
 
-  // unpack P = FFT(a + i b) into A = F(a), B = F(b) for kx < N/2
-  double2* __restrict__ w0 = static_cast<double2*>(a.w0);
-  double2* __restrict__ w1 = static_cast<double2*>(a.w1);
-  const int s = min(fx_shift_exact(ws.bits[NP], 62), 0);  // room for the sums
-  const FxScale out{sc.E - s - 1, sc.bad};
-  for (int w = tid; w < V * Nh; w += NT) {
-    const int v = w % V;
-    const int k = w / V;
-    fxc p[2] = {sm[PL::phys(k) * V + v], sm[PL::phys(k == 0 ? 0 : M - k) * V + v]};
-    fx_rescale<2>(p, s);
-    const size_t at = (size_t)k * M + z0 + v;
-    w0[at] = make_double2(fx_value(p[0].x + p[1].x, out), fx_value(p[0].y - p[1].y, out));
-    w1[at] = make_double2(fx_value(p[0].y + p[1].y, out), fx_value(p[1].x - p[0].x, out));
-  }
+  fx_rows_unpack<PL, V, NT>(a.w0, a.w1, sm, z0, tid, &ws, sc);
   if (stats) finish_stats<NT, false>(a, mx, acc, 0.0, M, tid, bk);
+}
+template <class PL, int V, int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB) k_row_fx(StepArgs a0) {
+  const Blk bk = hw_blk();
+  const StepArgs a = member_args(a0, sizeof(double2), bk.y);
+  row_fx_body<PL, V, NT>(a, a.w0, a.w1, bk);
 }
 
 // k_phys in fixed point: U-state rows -> physical u, v (statistics, optional
@@ -373,13 +385,41 @@ __global__ void __launch_bounds__(NT) k_phys_fx(StepArgs a0) {
   }
 }
 
-// 1 / d by two steps of Newton's iteration from the hardware's reciprocal
-// estimate (about 20 bits: each step doubles them).  d is finite and at least 1.
-__device__ __forceinline__ double newton_rcp(double d) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-  r = fma(r, fma(-d, r, 1.0), r);
-  return fma(r, fma(-d, r, 1.0), r);
+// Column kx of two planes into a raw tile, its largest high word in top[0].
+template <class PL, int NT>
+__device__ __forceinline__ void fx_column_load(fxc* sm, const void* p0, const void* p1, int kx, int tid, FxWords* ws) {
+  constexpr int M = PL::M, V = 2;
+  const double2* __restrict__ w0 = static_cast<const double2*>(p0) + (size_t)kx * M;
+  const double2* __restrict__ w1 = static_cast<const double2*>(p1) + (size_t)kx * M;
+  fx_words_clear<NT>(ws, tid);
+  __syncthreads();
+  unsigned top = 0;
+  constexpr int U = 8;  // loads in flight per thread
+  for (int w = tid; w < V * M; w += U * NT) {
+    double2 d[U];
+#pragma unroll
+    for (int c = 0; c < U; ++c)
+      if (w + c * NT < V * M) d[c] = (((w + c * NT) & 1) == 0 ? w0 : w1)[(w + c * NT) >> 1];
+#pragma unroll
+    for (int c = 0; c < U; ++c)
+      if (w + c * NT < V * M) {
+        sm[PL::phys((w + c * NT) >> 1) * V + ((w + c * NT) & 1)] = fx_raw(d[c]);
+        top = max(top, max(fx_top(d[c].x), fx_top(d[c].y)));
+      }
+  }
+  fx_note(top, &ws->top[0], tid);
+  __syncthreads();
+}
+// Forward passes 0 .. TO - 1 of a raw column tile (largest high word in top[0]).
+template <class PL, int NT, int TO>
+__device__ __forceinline__ FxScale fx_column_forward(fxc* sm, const int4* __restrict__ tw, int tid, FxWords* ws) {
+  const int emax = fx_emax(ws->top[0]);
+  FxScale sc{fx_exponent(emax, fx_bits(PL::R[0])), emax == 0x7ff};
+  fx_note(fx_pass<PL, 2, NT, 0, -1, false, true>(sm, tw, tid, emax, sc.bad), &ws->bits[0], tid);
+  sc.E += fx_gain<PL, 0>();
+  __syncthreads();
+  fx_dif<PL, 2, NT, -1, 1, TO, 0>(sm, tw, tid, ws, sc);
+  return sc;
 }
 
 // The inverse z-transform of a raw column tile (A tile of two lines in
@@ -419,11 +459,9 @@ __device__ __forceinline__ void fx_column_inverse(fxc* sm, const int4* __restric
 // reciprocals in four, the scale 1 / M^2 in the stage's weights, wave-number
 // products in integers (exact: N is at most 4096).  PERM and the stage flags as
 // k_col.  N=4096 1210 us (FP64 transforms: 4300), N=1024 78 us (317).
-template <class PL, int NT, bool PERM, int MINB>
-__global__ void __launch_bounds__(NT, MINB) k_col_fx(StepArgs a0) {
+template <class PL, int NT, bool PERM>
+__device__ __forceinline__ void col_fx_body(const StepArgs& a, void* d0, void* d1, const Blk bk) {
   static_assert(PL::M <= 6144, "K2 within 24 bits (fx_small)");
-  const Blk bk = hw_blk();
-  const StepArgs a = member_args(a0, sizeof(double2), bk.y);
   extern __shared__ __align__(128) unsigned char smraw[];
   __shared__ FxWords ws;
   fxc* sm = reinterpret_cast<fxc*>(smraw);
@@ -431,39 +469,13 @@ __global__ void __launch_bounds__(NT, MINB) k_col_fx(StepArgs a0) {
   const int tid = threadIdx.x;
   const int kx = bk.x;
   const int4* __restrict__ tw = static_cast<const int4*>(a.tw);
-  double2* __restrict__ w0 = static_cast<double2*>(a.w0);
-  double2* __restrict__ w1 = static_cast<double2*>(a.w1);
   double2* __restrict__ om =
       PERM ? static_cast<double2*>(a.om_p) + (size_t)kx * M : static_cast<double2*>(a.om) + (size_t)kx * N;
   double2* __restrict__ fm =
       PERM ? static_cast<double2*>(a.fm_p) + (size_t)kx * M : static_cast<double2*>(a.fnm1) + (size_t)kx * N;
-  fx_words_clear<NT>(&ws, tid);
-  __syncthreads();
-  {
-    unsigned top = 0;
-    constexpr int U = 8;  // loads in flight per thread
-    for (int w = tid; w < V * M; w += U * NT) {
-      double2 d[U];
-#pragma unroll
-      for (int c = 0; c < U; ++c)
-        if (w + c * NT < V * M) d[c] = (((w + c * NT) & 1) == 0 ? w0 : w1)[(size_t)kx * M + ((w + c * NT) >> 1)];
-#pragma unroll
-      for (int c = 0; c < U; ++c)
-        if (w + c * NT < V * M) {
-          sm[PL::phys((w + c * NT) >> 1) * V + ((w + c * NT) & 1)] = fx_raw(d[c]);
-          top = max(top, max(fx_top(d[c].x), fx_top(d[c].y)));
-        }
-    }
-    fx_note(top, &ws.top[0], tid);
-  }
+  fx_column_load<PL, NT>(sm, a.w0, a.w1, kx, tid, &ws);
   const ModeCoef<double> cf = col_coef<double>(a, N);
-  __syncthreads();
-  const int emax = fx_emax(ws.top[0]);
-  FxScale sc{fx_exponent(emax, fx_bits(PL::R[0])), emax == 0x7ff};
-  fx_note(fx_pass<PL, V, NT, 0, -1, false, true>(sm, tw, tid, emax, sc.bad), &ws.bits[0], tid);
-  sc.E += fx_gain<PL, 0>();
-  __syncthreads();
-  fx_dif<PL, V, NT, -1, 1, NP - 1, 0>(sm, tw, tid, &ws, sc);
+  FxScale sc = fx_column_forward<PL, NT, NP - 1>(sm, tw, tid, &ws);
 
   // last forward pass -> nonlinear term, update, inversion -> raw (u^, v^)
   {
@@ -563,8 +575,14 @@ __global__ void __launch_bounds__(NT, MINB) k_col_fx(StepArgs a0) {
     fx_note(top, &ws.top[1], tid);
     __syncthreads();
   }
-  fx_column_inverse<PL, NT, 1>(sm, tw, w0, w1, kx, tid, &ws);
+  fx_column_inverse<PL, NT, 1>(sm, tw, static_cast<double2*>(d0), static_cast<double2*>(d1), kx, tid, &ws);
   col_finish<NT>(a, tid, bk.nx);
+}
+template <class PL, int NT, bool PERM, int MINB>
+__global__ void __launch_bounds__(NT, MINB) k_col_fx(StepArgs a0) {
+  const Blk bk = hw_blk();
+  const StepArgs a = member_args(a0, sizeof(double2), bk.y);
+  col_fx_body<PL, NT, PERM>(a, a.w0, a.w1, bk);
 }
 
 // k_col_inv in fixed point: velocity low band (src, the om inversion, or a

@@ -10,6 +10,7 @@ using P96 = Plan<96, 16, 6>;
 using P192 = Plan<192, 16, 12>;
 using P384 = Plan<384, 16, 24>;
 using P384b = Plan<384, 24, 16>;
+using P384c = Plan<384, 4, 8, 12>;
 
 const RowKernels r32[] = {RowOf<float, P48, 4, 64>::make("8.6 V4x64"), RowOf<float, P48, 2, 64>::make("8.6 V2x64")};
 const ColKernels c32[] = {ColOf<float, P48, 64>::make("8.6 x64")};
@@ -33,8 +34,8 @@ const ColKernels c256[] = {ColOf<float, P384, 128>::make("16.24 x128"), ColOf<fl
                            ColOf<float, Rec<P384b>, 128, 2>::make("24.16r x128 hoist")};
 PAL_KERNEL_SET_ADJ(float, 0, 32, r32, c32, (AdjOf<float, P48, 4, 64, P48, 64>::get()))
 PAL_KERNEL_SET_ADJ(float, 0, 64, r64, c64, (AdjOf<float, P96, 4, 128, P96, 64>::get()))
-PAL_KERNEL_SET_ADJ(float, 0, 128, r128, c128, (AdjOf<float, P192, 4, 128, P192, 64>::get()))
-PAL_KERNEL_SET_ADJ(float, 0, 256, r256, c256, (AdjOf<float, P384, 4, 256, P384, 128>::get()))
+PAL_KERNEL_SET_ADJ(float, 0, 128, r128, c128, (AdjOf<float, Rec<P192>, 4, 128, Rec<P192>, 64>::get()))
+PAL_KERNEL_SET_ADJ(float, 0, 256, r256, c256, (AdjOf<float, Rec<P384>, 4, 128, Rec<P384c>, 96>::get()))
 }  // namespace
 
 const KernelSet* pal_kernels_f32_a(int N) {

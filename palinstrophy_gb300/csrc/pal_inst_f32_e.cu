@@ -9,6 +9,7 @@ using P576 = Plan<576, 24, 24>;
 using P576b = Plan<576, 6, 6, 16>;
 using P768 = Plan<768, 32, 24>;
 using P768b = Plan<768, 16, 2, 24>;
+using P768c = Plan<768, 8, 8, 12>;
 using P1152 = Plan<1152, 8, 6, 24>;
 using P1152b = Plan<1152, 12, 4, 24>;
 
@@ -50,7 +51,7 @@ const ColKernels c768[] = {ColOf<float, P1152, 256>::make("8.6.24 x256"), ColOf<
                            ColOf<float, Rec<P1152>, 256, 4>::make("8.6.24r x256 tma")};
 
 PAL_KERNEL_SET(float, 0, 384, r384, c384)
-PAL_KERNEL_SET_ADJ(float, 0, 512, r512, c512, (AdjOf<float, P768, 4, 256, P768, 128>::get()))
+PAL_KERNEL_SET_ADJ(float, 0, 512, r512, c512, (AdjOf<float, Rec<P768c>, 4, 384, Rec<P768c>, 192>::get()))
 PAL_KERNEL_SET(float, 0, 768, r768, c768)
 }  // namespace
 

@@ -1,23 +1,19 @@
 // FP64 candidates, N = 32 .. 512, with fixed-point transforms
-// (pal_fx_kernels.cuh); the adjoint's kernels transform in FP64.
+// (pal_fx_kernels.cuh, pal_fx_adjoint.cuh).
 #include "pal_launch.cuh"
 
 using namespace pal;
 
 namespace {
-using P48 = Plan<48, 3, 16>;
 using P48b = Plan<48, 6, 8>;
 using P48c = Plan<48, 4, 12>;
 using P96 = Plan<96, 6, 16>;
 using P96c = Plan<96, 8, 12>;
-using P192 = Plan<192, 12, 16>;
 using P192d = Plan<192, 4, 4, 12>;
-using P384 = Plan<384, 24, 16>;
 using P384b = Plan<384, 6, 8, 8>;
 using P384d = Plan<384, 4, 8, 12>;
 using P576 = Plan<576, 6, 6, 16>;
 using P576c = Plan<576, 6, 8, 12>;
-using P768 = Plan<768, 16, 3, 16>;
 using P768c = Plan<768, 12, 8, 8>;
 using P768d = Plan<768, 8, 8, 12>;
 
@@ -37,12 +33,12 @@ const RowKernels r512[] = {RowFxOf<P768d, 2, 192>::make("8.8.12 V2x192 fx"),
                            RowFxOf<P768c, 2, 192>::make("12.8.8 V2x192 fx")};
 const ColKernels c512[] = {ColFxOf<P768d, 192>::make("8.8.12 x192 fx")};
 
-PAL_KERNEL_SET_ADJ(double, 1, 32, r32, c32, (AdjOf<double, P48, 2, 64, P48, 64>::get()))
-PAL_KERNEL_SET_ADJ(double, 1, 64, r64, c64, (AdjOf<double, P96, 2, 64, P96, 64>::get()))
-PAL_KERNEL_SET_ADJ(double, 1, 128, r128, c128, (AdjOf<double, P192, 2, 128, P192, 64>::get()))
-PAL_KERNEL_SET_ADJ(double, 1, 256, r256, c256, (AdjOf<double, P384, 2, 256, P384, 128>::get()))
+PAL_KERNEL_SET_ADJ(double, 1, 32, r32, c32, (AdjOf<double, P48b, 2, 32, P48c, 32>::get()))
+PAL_KERNEL_SET_ADJ(double, 1, 64, r64, c64, (AdjOf<double, P96, 2, 64, P96c, 64>::get()))
+PAL_KERNEL_SET_ADJ(double, 1, 128, r128, c128, (AdjOf<double, P192d, 2, 96, P192d, 96>::get()))
+PAL_KERNEL_SET_ADJ(double, 1, 256, r256, c256, (AdjOf<double, P384b, 2, 128, P384b, 128>::get()))
 PAL_KERNEL_SET(double, 1, 384, r384, c384)
-PAL_KERNEL_SET_ADJ(double, 1, 512, r512, c512, (AdjOf<double, P768, 2, 256, P768, 128>::get()))
+PAL_KERNEL_SET_ADJ(double, 1, 512, r512, c512, (AdjOf<double, P768d, 2, 192, P768d, 192>::get()))
 }  // namespace
 
 const KernelSet* pal_kernels_f64_a(int N) {

@@ -8,11 +8,10 @@
 // and keeps the fastest (pal_autotune in pal_api.cu).
 #pragma once
 #include <algorithm>
+#include <atomic>
 #include <cstdlib>
 
-#include "pal_adjoint.cuh"
-#include "pal_fx_kernels.cuh"
-#include "pal_kernels.cuh"
+#include "pal_fx_adjoint.cuh"
 
 namespace pal {
 
@@ -50,17 +49,22 @@ struct ColKernels {
   int rp;                  // last radix of the plan (pad groups of the TMA column tile)
 };
 
-// Adjoint of one LS-IMEX-RK3 stage (pal_adjoint.cuh), on fixed plans.
+// Adjoint of LS-IMEX-RK3 stages (pal_adjoint.cuh, pal_fx_adjoint.cuh), on fixed
+// plans.  a.tw is the row or the column table as the kernel needs.
 struct AdjKernels {
   int tw_row_elems, tw_col_elems;
   cudaError_t (*configure)();
-  void (*col_in)(const StepArgs&, cudaStream_t);
-  void (*row)(const StepArgs&, cudaStream_t);
-  void (*col_out)(const StepArgs&, cudaStream_t);
-  void (*col_vel)(const StepArgs&, cudaStream_t);  // the stage's velocity planes from om_in
+  void (*vel)(const StepArgs&, cudaStream_t);      // om_p -> velocity planes y0, y1
+  void (*fwd_row)(const StepArgs&, cudaStream_t);  // y0, y1 -> product planes w0, w1
+  void (*fwd_col)(const StepArgs&, cudaStream_t);  // w0, w1, om_p, fm_p -> om_p, fm_p, y0, y1
+  void (*col)(const StepArgs&, cudaStream_t);      // F_ADJ_OUT / F_ADJ_IN on om_p = lam_om, fm_p = lam_f, w0, w1
+  void (*row)(const StepArgs&, cudaStream_t);      // lam planes w0, w1 with the velocity planes y0, y1
   void (*tw_row)(void* tw, cudaStream_t);
   void (*tw_col)(void* tw, cudaStream_t);
-  void (*seed)(const void* om, void* lom, void* lf, int N, double* loss_part, int blocks, cudaStream_t);
+  void (*seed)(const void* om, void* lom, void* lf, double* loss_part, cudaStream_t);  // N/2 partials
+  // columns between the natural and the adjoint plan's butterfly-major order (as ColKernels)
+  void (*to_perm)(const StepArgs&, cudaStream_t);
+  void (*from_perm)(const StepArgs&, cudaStream_t);
 };
 
 struct KernelSet {
@@ -157,9 +161,7 @@ struct RowOf {
       if (e != cudaSuccess) return e;
     }
     if (PF & 1) ahead = ((PF & 32) ? 2 : 1) * wave_blocks(k_row<T, PL, V, NT, PF>, NT, smem);
-    e = cudaFuncSetAttribute(k_phys<T, PL, V, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) phys_wave = wave_blocks(k_phys<T, PL, V, NT>, NT, smem);
-    return e;
+    return cudaFuncSetAttribute(k_phys<T, PL, V, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   }
   static void row(const StepArgs& a, cudaStream_t s) {
     StepArgs b = a;
@@ -170,10 +172,11 @@ struct RowOf {
   }
   // k_phys: one wave of blocks shared by the members, each looping over its
   // member's tiles
-  static inline int phys_wave = 0;
   static void phys(const StepArgs& a, cudaStream_t s) {
+    static std::atomic<int> wave{0};
     const int m = a.members > 1 ? a.members : 1;
-    k_phys<T, PL, V, NT><<<dim3(phys_blocks(PL::M / V, phys_wave, m), m), NT, smem, s>>>(a);
+    if (wave == 0) wave = wave_blocks(k_phys<T, PL, V, NT>, NT, smem);
+    k_phys<T, PL, V, NT><<<dim3(phys_blocks(PL::M / V, wave, m), m), NT, smem, s>>>(a);
   }
   static int blocks_per_sm() {
     int n = 0;
@@ -311,16 +314,15 @@ struct RowFxOf {
   static_assert(smem <= kSmemLimit && PL::M % V == 0 && NT % 32 == 0, "row tile, whole warps");
   static cudaError_t configure() {
     cudaError_t e = set_tile_smem(k_row_fx<FP, V, NT, MINB>, smem);
-    if (e == cudaSuccess) e = set_tile_smem(k_phys_fx<FP, V, NT>, smem);
-    if (e == cudaSuccess) phys_wave = wave_blocks(k_phys_fx<FP, V, NT>, NT, smem);
-    return e;
+    return e == cudaSuccess ? set_tile_smem(k_phys_fx<FP, V, NT>, smem) : e;
   }
-  static inline int phys_wave = 0;
   static dim3 grid(const StepArgs& a) { return dim3(PL::M / V, a.members > 1 ? a.members : 1); }
   static void row(const StepArgs& a, cudaStream_t s) { k_row_fx<FP, V, NT, MINB><<<grid(a), NT, smem, s>>>(a); }
   static void phys(const StepArgs& a, cudaStream_t s) {
+    static std::atomic<int> wave{0};
     const dim3 g = grid(a);
-    k_phys_fx<FP, V, NT><<<dim3(phys_blocks(g.x, phys_wave, g.y), g.y), NT, smem, s>>>(a);
+    if (wave == 0) wave = wave_blocks(k_phys_fx<FP, V, NT>, NT, smem);
+    k_phys_fx<FP, V, NT><<<dim3(phys_blocks(g.x, wave, g.y), g.y), NT, smem, s>>>(a);
   }
   static int blocks_per_sm() {
     int n = 0;
@@ -373,36 +375,81 @@ struct ColFxOf {
 
 template <typename T, class PLR, int V, int NTR, class PLC, int NTC>
 struct AdjOf {
-  static constexpr size_t smem_row = size_t(PLR::PADM) * V * sizeof(cplx<T>) * 2;
+  static constexpr bool FX = std::is_same_v<T, double>;
+  static constexpr size_t smem_fwd = size_t(PLR::PADM) * V * sizeof(cplx<T>);
+  static constexpr size_t smem_row = 2 * smem_fwd;  // the lam and the velocity tile
   static constexpr size_t smem_col = size_t(PLC::PADM) * 2 * sizeof(cplx<T>);
+  static constexpr size_t smem_perm = PermTile<T, PLC>::smem;
   static_assert(smem_row <= kSmemLimit && smem_col <= kSmemLimit, "adjoint tiles do not fit");
+  static constexpr int N = 2 * PLC::M / 3;
   static cudaError_t configure() {
-    cudaError_t e =
-        cudaFuncSetAttribute(k_adj_row<T, PLR, V, NTR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_adj_col_in<T, PLC, NTC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_col);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_adj_col_out<T, PLC, NTC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_col);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_col_inv<T, PLC, NTC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_col);
+    cudaError_t e;
+    if constexpr (FX) {
+      e = set_tile_smem(k_adj_row_fx<FxPlan<PLR>, V, NTR>, smem_row);
+      if (e == cudaSuccess) e = set_tile_smem(k_adj_fwd_row_fx<FxPlan<PLR>, V, NTR>, smem_fwd);
+      if (e == cudaSuccess) e = set_tile_smem(k_adj_col_fx<FxPlan<PLC>, NTC>, smem_col);
+      if (e == cudaSuccess) e = set_tile_smem(k_adj_fwd_col_fx<FxPlan<PLC>, NTC>, smem_col);
+      if (e == cudaSuccess) e = set_tile_smem(k_adj_vel_fx<FxPlan<PLC>, NTC>, smem_col);
+    } else {
+      e = set_tile_smem(k_adj_row<T, PLR, V, NTR>, smem_row);
+      if (e == cudaSuccess) e = set_tile_smem(k_adj_fwd_row<T, PLR, V, NTR>, smem_fwd);
+      if (e == cudaSuccess) e = set_tile_smem(k_adj_col<T, PLC, NTC>, smem_col);
+      if (e == cudaSuccess) e = set_tile_smem(k_adj_fwd_col<T, PLC, NTC>, smem_col);
+      if (e == cudaSuccess) e = set_tile_smem(k_adj_vel<T, PLC, NTC>, smem_col);
+    }
+    if (e == cudaSuccess) e = set_tile_smem(k_om_perm<T, PLC, true>, smem_perm);
+    if (e == cudaSuccess) e = set_tile_smem(k_om_perm<T, PLC, false>, smem_perm);
     return e;
   }
-  static void col_in(const StepArgs& a, cudaStream_t s) { k_adj_col_in<T, PLC, NTC><<<a.N / 2, NTC, smem_col, s>>>(a); }
+  static void vel(const StepArgs& a, cudaStream_t s) {
+    if constexpr (FX)
+      k_adj_vel_fx<FxPlan<PLC>, NTC><<<N / 2, NTC, smem_col, s>>>(a);
+    else
+      k_adj_vel<T, PLC, NTC><<<N / 2, NTC, smem_col, s>>>(a);
+  }
+  static void fwd_row(const StepArgs& a, cudaStream_t s) {
+    if constexpr (FX)
+      k_adj_fwd_row_fx<FxPlan<PLR>, V, NTR><<<PLR::M / V, NTR, smem_fwd, s>>>(a);
+    else
+      k_adj_fwd_row<T, PLR, V, NTR><<<PLR::M / V, NTR, smem_fwd, s>>>(a);
+  }
+  static void fwd_col(const StepArgs& a, cudaStream_t s) {
+    if constexpr (FX)
+      k_adj_fwd_col_fx<FxPlan<PLC>, NTC><<<N / 2, NTC, smem_col, s>>>(a);
+    else
+      k_adj_fwd_col<T, PLC, NTC><<<N / 2, NTC, smem_col, s>>>(a);
+  }
+  static void col(const StepArgs& a, cudaStream_t s) {
+    if constexpr (FX)
+      k_adj_col_fx<FxPlan<PLC>, NTC><<<N / 2, NTC, smem_col, s>>>(a);
+    else
+      k_adj_col<T, PLC, NTC><<<N / 2, NTC, smem_col, s>>>(a);
+  }
   static void row(const StepArgs& a, cudaStream_t s) {
-    k_adj_row<T, PLR, V, NTR><<<PLR::M / V, NTR, smem_row, s>>>(a);
+    if constexpr (FX)
+      k_adj_row_fx<FxPlan<PLR>, V, NTR><<<PLR::M / V, NTR, smem_row, s>>>(a);
+    else
+      k_adj_row<T, PLR, V, NTR><<<PLR::M / V, NTR, smem_row, s>>>(a);
   }
-  static void col_out(const StepArgs& a, cudaStream_t s) {
-    k_adj_col_out<T, PLC, NTC><<<a.N / 2, NTC, smem_col, s>>>(a);
+  static void seed(const void* om, void* lom, void* lf, double* loss_part, cudaStream_t s) {
+    k_adj_seed<T, PLC, 128><<<N / 2, 128, 0, s>>>(static_cast<const cplx<T>*>(om), static_cast<cplx<T>*>(lom),
+                                                  static_cast<cplx<T>*>(lf), loss_part);
   }
-  static void col_vel(const StepArgs& a, cudaStream_t s) { k_col_inv<T, PLC, NTC><<<a.N / 2, NTC, smem_col, s>>>(a); }
-  static void seed(const void* om, void* lom, void* lf, int N, double* loss_part, int blocks, cudaStream_t s) {
-    k_adj_seed<T><<<blocks, 256, 0, s>>>(static_cast<const cplx<T>*>(om), static_cast<cplx<T>*>(lom),
-                                         static_cast<cplx<T>*>(lf), N, loss_part);
+  static dim3 grid_perm(const StepArgs& a) { return dim3(N / 2, 1, (a.flags & F_NO_FM_IN) ? 1 : 2); }
+  static void to_perm(const StepArgs& a, cudaStream_t s) { k_om_perm<T, PLC, true><<<grid_perm(a), 256, smem_perm, s>>>(a); }
+  static void from_perm(const StepArgs& a, cudaStream_t s) {
+    k_om_perm<T, PLC, false><<<grid_perm(a), 256, smem_perm, s>>>(a);
   }
   static const AdjKernels* get() {
-    static const AdjKernels k = {PLR::TW_TOTAL,   PLC::TW_TOTAL, configure, col_in, row, col_out, col_vel,
-                                 launch_twiddles<T, PLR>, launch_twiddles<T, PLC>, seed};
-    return &k;
+    if constexpr (FX) {
+      static const AdjKernels k = {FxPlan<PLR>::TW_TOTAL, FxPlan<PLC>::TW_TOTAL, configure, vel, fwd_row, fwd_col, col, row,
+                                   launch_twiddles_fx<PLR>, launch_twiddles_fx<PLC>, seed, to_perm, from_perm};
+      return &k;
+    } else {
+      static const AdjKernels k = {PLR::TW_TOTAL, PLC::TW_TOTAL, configure, vel, fwd_row, fwd_col, col, row,
+                                   launch_twiddles<T, PLR>, launch_twiddles<T, PLC>, seed, to_perm, from_perm};
+      return &k;
+    }
   }
 };
 
