@@ -75,15 +75,16 @@ __device__ __forceinline__ AdjPair<T> adj_mode(int flags, cplx<T> lu, cplx<T> lv
   const int Nh = N >> 1;
   const T ax = T(kx), gz = T(z < Nh ? z : z - N);
   const T K2 = ax * ax + gz * gz;
+  constexpr T half = sizeof(T) == 4 ? T(0.5) : T(1);  // the FP32 row pass leaves twice the transforms
   C lw = lw_io;
   if (flags & F_ADJ_OUT) {
     if (kx >= 1) {
       // conj(-i gz/K2) w' lu + conj(i ax/K2) w' lv = i (gz w'/K2) lu - i (ax w'/K2) lv
-      const T ik = T(2) * adj_rcp(K2);
+      const T ik = T(2) * half * adj_rcp(K2);
       const T su = gz * ik, sv = ax * ik;
       lw = C{lw.x - su * lu.y + sv * lv.y, lw.y + su * lu.x - sv * lv.x};
     } else if (z >= 1) {
-      const T ig = T(1) / gz;  // conj(-i/gz) = i/gz
+      const T ig = half / gz;  // conj(-i/gz) = i/gz
       lw = C{lw.x - ig * lu.y, lw.y + ig * lu.x};
     }
   }

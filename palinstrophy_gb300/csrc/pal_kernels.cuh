@@ -5,7 +5,7 @@
 //   w0, w1   : [kx][z]  (N/2 lines of M)      the work planes, holding either
 //               U-state: velocity (u^, v^) after the inverse z-transform, or
 //               P-state: products after the forward x-transform,
-//                        A = F_x(u^2 - v^2), B = F_x(u v).
+//                        A = F_x(u^2 - v^2), B = F_x(u v) (in FP32 2A, 2B).
 // One stage of a step is two launches:
 //   k_row : per tile of V physical rows z: Hermitian-packed inverse x-FFT
 //           (u + i v), products, packed forward x-FFT, unpack A, B  (U -> P)
@@ -704,8 +704,9 @@ __device__ __forceinline__ void row_first_pass_tma(const StepArgs& a, cplx<T>* s
 // butterfly S - i at index R-1-j (for i = 0 in butterfly 0 at (R-j) mod R, for
 // i = S/2 in butterfly S/2 at R-1-j), so one thread transforms the pair
 // (q, S - q), or (0, S/2) for q = 0, and writes
-// A = (P[k] + conj P[M-k]) / 2 and B = (P[k] - conj P[M-k]) / (2i) for k < N/2
-// straight to the work planes.  Outputs with N/2 <= k <= M - N/2 are never formed.
+// 2 A = P[k] + conj P[M-k] and 2 B = (P[k] - conj P[M-k]) / i for k < N/2
+// straight to the work planes (the FP32 P-state holds twice the products'
+// transforms; the column pass's weight takes the factor back, exactly).  Outputs with N/2 <= k <= M - N/2 are never formed.
 template <typename T, class PL, int V, int NT>
 __device__ __forceinline__ void row_last_pass_paired(const StepArgs& a, cplx<T>* sm, int z0, int tid) {
   using C = cplx<T>;
@@ -747,15 +748,15 @@ __device__ __forceinline__ void row_last_pass_paired(const StepArgs& a, cplx<T>*
       if (j * S + S - 1 < Nh || k1 < Nh) {
         const C p = y1[j];
         const C c = self ? y1[(R - j) % R] : y2[R - 1 - j];
-        w0[(size_t)k1 * M + col] = C{T(0.5) * (p.x + c.x), T(0.5) * (p.y - c.y)};
-        w1[(size_t)k1 * M + col] = C{T(0.5) * (p.y + c.y), T(-0.5) * (p.x - c.x)};
+        w0[(size_t)k1 * M + col] = C{p.x + c.x, p.y - c.y};
+        w1[(size_t)k1 * M + col] = C{p.y + c.y, c.x - p.x};
       }
       const int k2 = i2 + j * S;
       if (j * S + S - 1 < Nh || k2 < Nh) {
         const C p = y2[j];
         const C c = self ? y2[R - 1 - j] : y1[R - 1 - j];
-        w0[(size_t)k2 * M + col] = C{T(0.5) * (p.x + c.x), T(0.5) * (p.y - c.y)};
-        w1[(size_t)k2 * M + col] = C{T(0.5) * (p.y + c.y), T(-0.5) * (p.x - c.x)};
+        w0[(size_t)k2 * M + col] = C{p.x + c.x, p.y - c.y};
+        w1[(size_t)k2 * M + col] = C{p.y + c.y, c.x - p.x};
       }
     }
   }
@@ -807,11 +808,11 @@ __device__ __forceinline__ void row_last_pass_tma(const StepArgs& a, cplx<T>* sm
 #pragma unroll
   for (int j = 0; j < JN; ++j) {
     const C p1 = y1[j], c1 = self ? y1[(R - j) % R] : y2[R - 1 - j];
-    A1[j] = C{T(0.5) * (p1.x + c1.x), T(0.5) * (p1.y - c1.y)};
-    B1[j] = C{T(0.5) * (p1.y + c1.y), T(-0.5) * (p1.x - c1.x)};
+    A1[j] = C{p1.x + c1.x, p1.y - c1.y};
+    B1[j] = C{p1.y + c1.y, c1.x - p1.x};
     const C p2 = y2[j], c2 = self ? y2[R - 1 - j] : y1[R - 1 - j];
-    A2[j] = C{T(0.5) * (p2.x + c2.x), T(0.5) * (p2.y - c2.y)};
-    B2[j] = C{T(0.5) * (p2.y + c2.y), T(-0.5) * (p2.x - c2.x)};
+    A2[j] = C{p2.x + c2.x, p2.y - c2.y};
+    B2[j] = C{p2.y + c2.y, c2.x - p2.x};
   }
   __syncthreads();  // every read of the tile is done: reuse it as the staging area
   C* stg = sm;      // [plane][k < N/2][v]
@@ -940,28 +941,12 @@ __device__ __forceinline__ void row_body(const StepArgs& a0, const TmaMaps& maps
   const bool stats = (a.flags & (ENS ? (F_STATS | F_STATS_MAX) : F_STATS)) != 0;
   T mx = T(0), acc = T(0);
   row_products<T, PL, V, NT>(sm, tid, stats, mx, acc);
-  if constexpr (sizeof(C) == 8) {
-    dit_range<T, PL, V, NT, -1, PL::NP - 2, 1>(sm, tw, tid);
-    if constexpr ((PF & 4) != 0)
-      row_last_pass_tma<T, PL, V, NT>(a, sm, z0, tid, maps, bk.y);
-    else
-      row_last_pass_paired<T, PL, V, NT>(a, sm, z0, tid);
-  } else {
-    dit_range<T, PL, V, NT, -1, PL::NP - 2, 0>(sm, tw, tid);
-    // unpack P = FFT(a + i b) into A = F(a), B = F(b) for kx < N/2 and store
-    C* __restrict__ w0 = static_cast<C*>(a.w0);
-    C* __restrict__ w1 = static_cast<C*>(a.w1);
-    constexpr int Nh = M / 3;
-    for (int w = tid; w < V * Nh; w += NT) {
-      const int v = w % V;
-      const int k = w / V;
-      const C p = sm[PL::phys(k) * V + v];
-      const C q = sm[PL::phys(k == 0 ? 0 : M - k) * V + v];
-      w0[(size_t)k * M + z0 + v] = C{T(0.5) * (p.x + q.x), T(0.5) * (p.y - q.y)};
-      w1[(size_t)k * M + z0 + v] = C{T(0.5) * (p.y + q.y), T(-0.5) * (p.x - q.x)};
-    }
-  }
-  if constexpr (ENS && sizeof(T) == 4) {
+  dit_range<T, PL, V, NT, -1, PL::NP - 2, 1>(sm, tw, tid);
+  if constexpr ((PF & 4) != 0)
+    row_last_pass_tma<T, PL, V, NT>(a, sm, z0, tid, maps, bk.y);
+  else
+    row_last_pass_paired<T, PL, V, NT>(a, sm, z0, tid);
+  if constexpr (ENS) {
     if (a.flags & F_STATS)
       finish_stats<NT, false>(a, double(mx), double(acc), 0.0, M, tid, bk);
     else if (a.flags & F_STATS_MAX)
@@ -1096,7 +1081,7 @@ __device__ __forceinline__ ModeCoef<T> col_coef(const StepArgs& a, int N) {
   cf.c2 = T(c2);
   cf.c3 = T(c3);
   const T m32 = T(1.5) * T(N);
-  cf.divxz = T(1) / (m32 * m32);
+  cf.divxz = (sizeof(T) == 4 ? T(0.5) : T(1)) / (m32 * m32);  // FP32: the P-state is doubled
   return cf;
 }
 

@@ -353,8 +353,8 @@ __device__ __forceinline__ void split_first_pass(const StepArgs& a, float2* sm, 
 
 // Unpack of output row k from P[k] (p) and P[M - k] (c), as row_last_pass_tma.
 __device__ __forceinline__ void split_unpack(float2 p, float2 c, float2& A, float2& B) {
-  A = float2{0.5f * (p.x + c.x), 0.5f * (p.y - c.y)};
-  B = float2{0.5f * (p.y + c.y), -0.5f * (p.x - c.x)};
+  A = float2{p.x + c.x, p.y - c.y};
+  B = float2{p.y + c.y, c.x - p.x};
 }
 // P[k] and P[M - k] from own / peer G values: g0 = G_0[k], g1 = G_1[k],
 // h0 = G_0[M/2 - k], h1 = G_1[M/2 - k], w = e^{-2 pi i k / M}.
