@@ -122,6 +122,7 @@ __device__ __forceinline__ void for_column(int tid, F&& f) {
 
 template <typename T, class PL, int NT>
 __global__ void __launch_bounds__(NT) k_adj_col(StepArgs a) {
+  pdl_wait();
   using C = cplx<T>;
   extern __shared__ __align__(128) unsigned char smraw[];
   C* sm = reinterpret_cast<C*>(smraw);
@@ -161,6 +162,7 @@ __global__ void __launch_bounds__(NT) k_adj_col(StepArgs a) {
 // butterflies in the last inverse pass, where the pointwise step happens.
 template <typename T, class PL, int V, int NT>
 __global__ void __launch_bounds__(NT) k_adj_row(StepArgs a) {
+  pdl_wait();
   using C = cplx<T>;
   extern __shared__ __align__(128) unsigned char smraw[];
   C* lam = reinterpret_cast<C*>(smraw);
@@ -208,6 +210,7 @@ __global__ void __launch_bounds__(NT) k_adj_row(StepArgs a) {
 // product planes (w0, w1) ...
 template <typename T, class PL, int V, int NT>
 __global__ void __launch_bounds__(NT) k_adj_fwd_row(StepArgs a) {
+  pdl_wait();
   extern __shared__ __align__(128) unsigned char smraw[];
   cplx<T>* sm = reinterpret_cast<cplx<T>*>(smraw);
   const int tid = threadIdx.x, z0 = blockIdx.x * V;
@@ -227,6 +230,7 @@ __global__ void __launch_bounds__(NT) k_adj_fwd_row(StepArgs a) {
 // planes (y0, y1).
 template <typename T, class PL, int NT>
 __global__ void __launch_bounds__(NT) k_adj_fwd_col(StepArgs a) {
+  pdl_wait();
   using C = cplx<T>;
   extern __shared__ __align__(128) unsigned char smraw[];
   C* sm = reinterpret_cast<C*>(smraw);
@@ -282,6 +286,7 @@ __device__ __forceinline__ cplx<T> adj_velocity(cplx<T> o, int kx, int z, int N,
 // om -> velocity planes (y0, y1).
 template <typename T, class PL, int NT>
 __global__ void __launch_bounds__(NT) k_adj_vel(StepArgs a) {
+  pdl_wait();
   using C = cplx<T>;
   extern __shared__ __align__(128) unsigned char smraw[];
   C* sm = reinterpret_cast<C*>(smraw);

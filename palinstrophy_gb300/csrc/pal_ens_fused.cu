@@ -93,11 +93,10 @@ struct FusedOf {
   static constexpr size_t smem_col = std::max({Ss::smem_col...});
   static constexpr size_t smem_perm = std::max({Ss::smem_perm...});
   static_assert(smem_row <= kSmemLimit && smem_col <= kSmemLimit, "fused tiles fit in shared memory");
-  // row and statistics passes run NT threads per block, the column and layout
-  // passes NTC
+  // row and statistics passes run NT threads per block, the column passes NTC
   template <int PASS>
   static constexpr int threads() {
-    return (PASS == P_ROW || PASS == P_PHYS) ? NT : NTC;
+    return (PASS == P_ROW || PASS == P_PHYS) ? NT : (PASS == P_TO || PASS == P_FROM) ? 128 : NTC;
   }
   template <int PASS>
   static void launch(const FusedArgs& f, int blocks, size_t smem, cudaStream_t s) {
@@ -121,8 +120,8 @@ struct FusedOf {
               {(const void*)k_ens_fused<P_COL, NTC, Ss...>, smem_col},
               {(const void*)k_ens_fused<P_COL_QM, NTC, Ss...>, smem_col},
               {(const void*)k_ens_fused<P_PHYS, NT, Ss...>, smem_row},
-              {(const void*)k_ens_fused<P_TO, NTC, Ss...>, smem_perm},
-              {(const void*)k_ens_fused<P_FROM, NTC, Ss...>, smem_perm}};
+              {(const void*)k_ens_fused<P_TO, 128, Ss...>, smem_perm},
+              {(const void*)k_ens_fused<P_FROM, 128, Ss...>, smem_perm}};
     for (const auto& k : ks) {
       cudaError_t e = cudaFuncSetAttribute(k.k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem);
       if (e != cudaSuccess) return e;

@@ -8,6 +8,7 @@ namespace pal {
 
 template <class PL, int NT>
 __global__ void __launch_bounds__(NT) k_adj_col_fx(StepArgs a) {
+  pdl_wait();
   extern __shared__ __align__(128) unsigned char smraw[];
   __shared__ FxWords ws;
   fxc* sm = reinterpret_cast<fxc*>(smraw);
@@ -52,6 +53,7 @@ __global__ void __launch_bounds__(NT) k_adj_col_fx(StepArgs a) {
 
 template <class PL, int V, int NT>
 __global__ void __launch_bounds__(NT) k_adj_row_fx(StepArgs a) {
+  pdl_wait();
   extern __shared__ __align__(128) unsigned char smraw[];
   __shared__ FxWords wl, wv;
   fxc* lam = reinterpret_cast<fxc*>(smraw);
@@ -96,16 +98,19 @@ __global__ void __launch_bounds__(NT) k_adj_row_fx(StepArgs a) {
 
 template <class PL, int V, int NT>
 __global__ void __launch_bounds__(NT) k_adj_fwd_row_fx(StepArgs a) {
+  pdl_wait();
   row_fx_body<PL, V, NT>(a, a.y0, a.y1, hw_blk());
 }
 
 template <class PL, int NT>
 __global__ void __launch_bounds__(NT) k_adj_fwd_col_fx(StepArgs a) {
+  pdl_wait();
   col_fx_body<PL, NT, true>(a, const_cast<void*>(a.y0), const_cast<void*>(a.y1), hw_blk());
 }
 
 template <class PL, int NT>
 __global__ void __launch_bounds__(NT) k_adj_vel_fx(StepArgs a) {
+  pdl_wait();
   extern __shared__ __align__(128) unsigned char smraw[];
   __shared__ FxWords ws;
   fxc* sm = reinterpret_cast<fxc*>(smraw);

@@ -149,6 +149,24 @@ __device__ __forceinline__ StepArgs member_args(const StepArgs& a, size_t esz) {
 
 constexpr double kPi = 3.14159265358979323846;
 
+// First statement of a kernel that launch_pdl may launch early: the kernel before
+// it in the stream has finished and its writes are visible, and the next one's
+// blocks may be brought in as this grid's last ones start.  Nothing of the work
+// moves before it.  Kernels that are not launched early leave it out: with many
+// short blocks it costs 2 % of the pass.
+template <bool EARLY = true>
+__device__ __forceinline__ void pdl_wait() {
+  if constexpr (EARLY) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  }
+}
+constexpr int kEarlyM = 2304;
+template <class PL>
+constexpr bool early_plan() {
+  return PL::M >= kEarlyM;
+}
+
 // --------------------------------------------------------------------------
 // Block reductions (deterministic: fixed tree order)
 template <int NT, int K>
@@ -958,6 +976,7 @@ __device__ __forceinline__ void row_body(const StepArgs& a0, const TmaMaps& maps
 template <typename T, class PL, int V, int NT, int PF>
 __global__ void __launch_bounds__(NT, (PF & 16) ? row_tiles_per_sm<T, PL, V>() : 0)
     k_row(StepArgs a0, const __grid_constant__ TmaMaps maps) {
+  pdl_wait<early_plan<PL>()>();
   row_body<T, PL, V, NT, PF>(a0, maps, hw_blk());
 }
 
@@ -1029,6 +1048,7 @@ __device__ __forceinline__ void phys_body(const StepArgs& a0, const Blk bk) {
 }
 template <typename T, class PL, int V, int NT>
 __global__ void __launch_bounds__(NT) k_phys(StepArgs a0) {
+  pdl_wait<early_plan<PL>()>();
   phys_body<T, PL, V, NT>(a0, hw_blk());
 }
 
@@ -1443,6 +1463,7 @@ __device__ __forceinline__ void col_body(const StepArgs& a0, const Blk bk) {
 }
 template <typename T, class PL, int NT, int PREF, bool PERM, bool QM = true>
 __global__ void __launch_bounds__(NT) k_col(StepArgs a0) {
+  pdl_wait<early_plan<PL>()>();
   col_body<T, PL, NT, PREF, PERM, QM>(a0, hw_blk());
 }
 
@@ -1591,6 +1612,7 @@ __device__ __forceinline__ void col_dit_planar(cplx<T>* sm, const cplx<T>* __res
 // (col_pass_planar_dual).
 template <typename T, class PL, int NT, bool QM, int MINB = 0, bool DUAL = false>
 __global__ void __launch_bounds__(NT, MINB) k_col_tma(StepArgs a0, const __grid_constant__ TmaMaps maps) {
+  pdl_wait<early_plan<PL>()>();
   using C = cplx<T>;
   using CP = ColPlanar<PL>;
   static_assert(sizeof(C) == 8 && CP::fits, "FP32 planes of whole pad groups and boxes");
@@ -1677,10 +1699,16 @@ __device__ __forceinline__ void om_perm_column(cplx<T>* sm, cplx<T>* __restrict_
     for (int z = tid; z < N; z += NT) sm[PT::slot(z)] = nat[z];
     __syncthreads();
   }
-  for (int b = tid; b < FSTEP; b += NT) {
+  // a thread takes one butterfly's entries, every G-th of them where there are
+  // fewer butterflies than threads (small grids)
+  constexpr int G = FSTEP >= NT ? 1 : NT / FSTEP;
+  for (int w = tid; w < G * FSTEP; w += NT) {
+    const int b = w % FSTEP, j0 = w / FSTEP;
     const int fb = PL::freq(b * RP);
 #pragma unroll
-    for (int j = 0; j < RP; ++j) {
+    for (int jj = 0; jj < RP; jj += G) {
+      const int j = G == 1 ? jj : jj + j0;
+      if (RP % G != 0 && j >= RP) continue;
       if (BAND_CT && j >= RP / 3 && j < 2 * (RP / 3)) continue;
       const int f = fb + j * FSTEP;
       if (!BAND_CT && f >= Nh && f < N) continue;
@@ -1713,8 +1741,9 @@ __device__ __forceinline__ void om_perm_body(const StepArgs& a0, const Blk bk, b
     om_perm_column<T, PL, TO_PERM, NT>(sm, static_cast<C*>(a.fnm1) + (size_t)kx * N,
                                        static_cast<C*>(a.fm_p) + (size_t)kx * M, threadIdx.x);
 }
-template <typename T, class PL, bool TO_PERM>
+template <typename T, class PL, bool TO_PERM, bool EARLY>
 __global__ void __launch_bounds__(256) k_om_perm(StepArgs a0) {
+  pdl_wait<EARLY>();
   om_perm_body<T, PL, TO_PERM, 256>(a0, hw_blk(), blockIdx.z == 0, blockIdx.z == 1);
 }
 
@@ -1767,6 +1796,7 @@ __device__ __forceinline__ cplx<T> col_inv_value(const StepArgs& a, int kx, int 
 }
 template <typename T, class PL, int NT>
 __global__ void __launch_bounds__(NT) k_col_inv(StepArgs a0) {
+  pdl_wait<early_plan<PL>()>();
   using C = cplx<T>;
   const StepArgs a = member_args(a0, sizeof(C));
   extern __shared__ __align__(128) unsigned char smraw[];

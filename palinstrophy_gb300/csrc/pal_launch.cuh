@@ -108,6 +108,31 @@ bool encode_row_maps(TmaMaps* out, void* w0, void* w1, int N, int V, int members
 // box, so one box row is a padded group of ColPlanar.
 bool encode_col_maps(TmaMaps* out, void* w0, void* w1, int N, int RP, int members);
 
+// Launch of a kernel that begins with pdl_wait() (its EARLY the same): with
+// EARLY the stream may bring its blocks onto the GPU while the previous kernel's
+// last ones run, which saves the launch between two kernels (about 1.5 us).  The
+// blocks that wait hold their SM's registers and shared memory, though, and
+// where several streams share the GPU with small kernels that costs more: three
+// N=256 FP64 fields side by side took 372 us a call with it and 293 without.  So
+// early launches are for FP32 passes of several waves (kEarlyM: N=4096 RK3 3.50
+// ms for four steps, 3.55 without; one N=1536 field alone 1.77 ms for ten, 1.92
+// without) and for the adjoint's short dependent launches (N=512 gradient 3.82
+// ms, 4.36 without).
+template <bool EARLY, class... P, class... A>
+inline void launch_pdl(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, const A&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = EARLY ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, args...);  // an error stays for the caller's cudaGetLastError
+}
+
 template <typename T, class PL>
 void launch_twiddles(void* tw, cudaStream_t s) {
   k_twiddles<T, PL><<<(PL::TW_TOTAL + 255) / 256, 256, 0, s>>>(static_cast<cplx<T>*>(tw));
@@ -144,6 +169,7 @@ __host__ __device__ inline void rk3_stage_flags(StepArgs& a, int s, const double
 
 template <typename T, class PL, int V, int NT, int PF = 0>
 struct RowOf {
+  static constexpr bool EARLY = early_plan<PL>();
   static constexpr size_t smem = std::max(size_t(PL::PADM) * V * sizeof(cplx<T>), size_t(2) * NT * sizeof(double));
   static_assert(smem <= kSmemLimit, "row tile does not fit in shared memory");
   static_assert(PL::M % V == 0, "row tile must divide M");
@@ -167,8 +193,7 @@ struct RowOf {
     StepArgs b = a;
     b.ahead = ahead;
     static const TmaMaps none{};
-    k_row<T, PL, V, NT, PF><<<dim3(PL::M / V, a.members > 1 ? a.members : 1), NT, smem, s>>>(
-        b, ((PF & 12) != 0 && a.tmaps) ? *a.tmaps : none);
+    launch_pdl<EARLY>(k_row<T, PL, V, NT, PF>, dim3(PL::M / V, a.members > 1 ? a.members : 1), NT, smem, s, b, ((PF & 12) != 0 && a.tmaps) ? *a.tmaps : none);
   }
   // k_phys: one wave of blocks shared by the members, each looping over its
   // member's tiles
@@ -176,7 +201,7 @@ struct RowOf {
     static std::atomic<int> wave{0};
     const int m = a.members > 1 ? a.members : 1;
     if (wave == 0) wave = wave_blocks(k_phys<T, PL, V, NT>, NT, smem);
-    k_phys<T, PL, V, NT><<<dim3(phys_blocks(PL::M / V, wave, m), m), NT, smem, s>>>(a);
+    launch_pdl<EARLY>(k_phys<T, PL, V, NT>, dim3(phys_blocks(PL::M / V, wave, m), m), NT, smem, s, a);
   }
   static int blocks_per_sm() {
     int n = 0;
@@ -190,6 +215,7 @@ struct RowOf {
 
 template <typename T, class PL, int NT, int PREF = 0>
 struct ColOf {
+  static constexpr bool EARLY = early_plan<PL>();
   // PREF 4: the butterfly-major pass is k_col_tma (planar tile, TMA bulk
   // copies of the planes); the natural-order pass is the plain k_col.
   // PREF 5 / 6: the same with registers capped for three / two blocks per SM.
@@ -236,14 +262,14 @@ struct ColOf {
                                cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
       if (e != cudaSuccess) return e;
     }
-    e = cudaFuncSetAttribute(k_om_perm<T, PL, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_perm);
+    e = cudaFuncSetAttribute(k_om_perm<T, PL, true, EARLY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_perm);
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_om_perm<T, PL, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_perm);
+    e = cudaFuncSetAttribute(k_om_perm<T, PL, false, EARLY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_perm);
     if (e != cudaSuccess) return e;
     return cudaFuncSetAttribute(k_col_inv<T, PL, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_inv);
   }
   static dim3 grid(const StepArgs& a) { return dim3(a.N / 2, a.members > 1 ? a.members : 1); }
-  static void col(const StepArgs& a, cudaStream_t s) { k_col<T, PL, NT, BASE, false><<<grid(a), NT, smem, s>>>(a); }
+  static void col(const StepArgs& a, cudaStream_t s) { launch_pdl<EARLY>(k_col<T, PL, NT, BASE, false>, grid(a), NT, smem, s, a); }
   // RK3 stages carrying the combined term run the flag-aware instantiation;
   // every other butterfly-major column pass runs the plain update
   static void col_perm(const StepArgs& a, cudaStream_t s) {
@@ -251,15 +277,15 @@ struct ColOf {
       static const TmaMaps none{};
       const TmaMaps& m = a.cmaps ? *a.cmaps : none;
       if (a.flags & (F_Q_IN | F_Q_OUT | F_NO_FM_IN))
-        k_col_tma<T, PL, NT, true, MINB, DUAL><<<grid(a), NT, smem_tma, s>>>(a, m);
+        launch_pdl<EARLY>(k_col_tma<T, PL, NT, true, MINB, DUAL>, grid(a), NT, smem_tma, s, a, m);
       else
-        k_col_tma<T, PL, NT, false, MINB, DUAL><<<grid(a), NT, smem_tma, s>>>(a, m);
+        launch_pdl<EARLY>(k_col_tma<T, PL, NT, false, MINB, DUAL>, grid(a), NT, smem_tma, s, a, m);
       return;
     }
     if (a.flags & (F_Q_IN | F_Q_OUT | F_NO_FM_IN))
-      k_col<T, PL, NT, PERM_PREF, true, true><<<grid(a), NT, smem_inv, s>>>(a);
+      launch_pdl<EARLY>(k_col<T, PL, NT, PERM_PREF, true, true>, grid(a), NT, smem_inv, s, a);
     else
-      k_col<T, PL, NT, PERM_PREF, true, false><<<grid(a), NT, smem_inv, s>>>(a);
+      launch_pdl<EARLY>(k_col<T, PL, NT, PERM_PREF, true, false>, grid(a), NT, smem_inv, s, a);
   }
   static constexpr size_t smem_perm = PermTile<T, PL>::smem;  // one om or fnm1 column
   static_assert(smem_perm <= kSmemLimit, "om / fnm1 column does not fit in shared memory");
@@ -268,13 +294,13 @@ struct ColOf {
     return dim3(g.x, g.y, (a.flags & F_NO_FM_IN) ? 1 : 2);
   }
   static void to_perm(const StepArgs& a, cudaStream_t s) {
-    k_om_perm<T, PL, true><<<grid_perm(a), 256, smem_perm, s>>>(a);
+    launch_pdl<EARLY>(k_om_perm<T, PL, true, EARLY>, grid_perm(a), 256, smem_perm, s, a);
   }
   static void from_perm(const StepArgs& a, cudaStream_t s) {
-    k_om_perm<T, PL, false><<<grid_perm(a), 256, smem_perm, s>>>(a);
+    launch_pdl<EARLY>(k_om_perm<T, PL, false, EARLY>, grid_perm(a), 256, smem_perm, s, a);
   }
   static void col_inv(const StepArgs& a, cudaStream_t s) {
-    k_col_inv<T, PL, NT><<<dim3(a.N / 2, a.members > 1 ? a.members : 1), NT, smem_inv, s>>>(a);
+    launch_pdl<EARLY>(k_col_inv<T, PL, NT>, dim3(a.N / 2, a.members > 1 ? a.members : 1), NT, smem_inv, s, a);
   }
   static int blocks_per_sm() {
     int n = 0;
@@ -344,9 +370,9 @@ struct ColFxOf {
     if (e == cudaSuccess) e = set_tile_smem(k_col_fx<FP, NT, true, MINB>, smem);
     if (e == cudaSuccess) e = set_tile_smem(k_col_inv_fx<FP, NT>, smem);
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_om_perm<double, PL, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_perm);
+      e = cudaFuncSetAttribute(k_om_perm<double, PL, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_perm);
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_om_perm<double, PL, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_perm);
+      e = cudaFuncSetAttribute(k_om_perm<double, PL, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_perm);
     return e;
   }
   static dim3 grid(const StepArgs& a) { return dim3(a.N / 2, a.members > 1 ? a.members : 1); }
@@ -358,10 +384,10 @@ struct ColFxOf {
   static void col_perm(const StepArgs& a, cudaStream_t s) { k_col_fx<FP, NT, true, MINB><<<grid(a), NT, smem, s>>>(a); }
   static void col_inv(const StepArgs& a, cudaStream_t s) { k_col_inv_fx<FP, NT><<<grid(a), NT, smem, s>>>(a); }
   static void to_perm(const StepArgs& a, cudaStream_t s) {
-    k_om_perm<double, PL, true><<<grid_perm(a), 256, smem_perm, s>>>(a);
+    k_om_perm<double, PL, true, false><<<grid_perm(a), 256, smem_perm, s>>>(a);
   }
   static void from_perm(const StepArgs& a, cudaStream_t s) {
-    k_om_perm<double, PL, false><<<grid_perm(a), 256, smem_perm, s>>>(a);
+    k_om_perm<double, PL, false, false><<<grid_perm(a), 256, smem_perm, s>>>(a);
   }
   static int blocks_per_sm() {
     int n = 0;
@@ -397,48 +423,48 @@ struct AdjOf {
       if (e == cudaSuccess) e = set_tile_smem(k_adj_fwd_col<T, PLC, NTC>, smem_col);
       if (e == cudaSuccess) e = set_tile_smem(k_adj_vel<T, PLC, NTC>, smem_col);
     }
-    if (e == cudaSuccess) e = set_tile_smem(k_om_perm<T, PLC, true>, smem_perm);
-    if (e == cudaSuccess) e = set_tile_smem(k_om_perm<T, PLC, false>, smem_perm);
+    if (e == cudaSuccess) e = set_tile_smem(k_om_perm<T, PLC, true, true>, smem_perm);
+    if (e == cudaSuccess) e = set_tile_smem(k_om_perm<T, PLC, false, true>, smem_perm);
     return e;
   }
   static void vel(const StepArgs& a, cudaStream_t s) {
     if constexpr (FX)
-      k_adj_vel_fx<FxPlan<PLC>, NTC><<<N / 2, NTC, smem_col, s>>>(a);
+      launch_pdl<true>(k_adj_vel_fx<FxPlan<PLC>, NTC>, N / 2, NTC, smem_col, s, a);
     else
-      k_adj_vel<T, PLC, NTC><<<N / 2, NTC, smem_col, s>>>(a);
+      launch_pdl<true>(k_adj_vel<T, PLC, NTC>, N / 2, NTC, smem_col, s, a);
   }
   static void fwd_row(const StepArgs& a, cudaStream_t s) {
     if constexpr (FX)
-      k_adj_fwd_row_fx<FxPlan<PLR>, V, NTR><<<PLR::M / V, NTR, smem_fwd, s>>>(a);
+      launch_pdl<true>(k_adj_fwd_row_fx<FxPlan<PLR>, V, NTR>, PLR::M / V, NTR, smem_fwd, s, a);
     else
-      k_adj_fwd_row<T, PLR, V, NTR><<<PLR::M / V, NTR, smem_fwd, s>>>(a);
+      launch_pdl<true>(k_adj_fwd_row<T, PLR, V, NTR>, PLR::M / V, NTR, smem_fwd, s, a);
   }
   static void fwd_col(const StepArgs& a, cudaStream_t s) {
     if constexpr (FX)
-      k_adj_fwd_col_fx<FxPlan<PLC>, NTC><<<N / 2, NTC, smem_col, s>>>(a);
+      launch_pdl<true>(k_adj_fwd_col_fx<FxPlan<PLC>, NTC>, N / 2, NTC, smem_col, s, a);
     else
-      k_adj_fwd_col<T, PLC, NTC><<<N / 2, NTC, smem_col, s>>>(a);
+      launch_pdl<true>(k_adj_fwd_col<T, PLC, NTC>, N / 2, NTC, smem_col, s, a);
   }
   static void col(const StepArgs& a, cudaStream_t s) {
     if constexpr (FX)
-      k_adj_col_fx<FxPlan<PLC>, NTC><<<N / 2, NTC, smem_col, s>>>(a);
+      launch_pdl<true>(k_adj_col_fx<FxPlan<PLC>, NTC>, N / 2, NTC, smem_col, s, a);
     else
-      k_adj_col<T, PLC, NTC><<<N / 2, NTC, smem_col, s>>>(a);
+      launch_pdl<true>(k_adj_col<T, PLC, NTC>, N / 2, NTC, smem_col, s, a);
   }
   static void row(const StepArgs& a, cudaStream_t s) {
     if constexpr (FX)
-      k_adj_row_fx<FxPlan<PLR>, V, NTR><<<PLR::M / V, NTR, smem_row, s>>>(a);
+      launch_pdl<true>(k_adj_row_fx<FxPlan<PLR>, V, NTR>, PLR::M / V, NTR, smem_row, s, a);
     else
-      k_adj_row<T, PLR, V, NTR><<<PLR::M / V, NTR, smem_row, s>>>(a);
+      launch_pdl<true>(k_adj_row<T, PLR, V, NTR>, PLR::M / V, NTR, smem_row, s, a);
   }
   static void seed(const void* om, void* lom, void* lf, double* loss_part, cudaStream_t s) {
     k_adj_seed<T, PLC, 128><<<N / 2, 128, 0, s>>>(static_cast<const cplx<T>*>(om), static_cast<cplx<T>*>(lom),
                                                   static_cast<cplx<T>*>(lf), loss_part);
   }
   static dim3 grid_perm(const StepArgs& a) { return dim3(N / 2, 1, (a.flags & F_NO_FM_IN) ? 1 : 2); }
-  static void to_perm(const StepArgs& a, cudaStream_t s) { k_om_perm<T, PLC, true><<<grid_perm(a), 256, smem_perm, s>>>(a); }
+  static void to_perm(const StepArgs& a, cudaStream_t s) { launch_pdl<true>(k_om_perm<T, PLC, true, true>, grid_perm(a), 256, smem_perm, s, a); }
   static void from_perm(const StepArgs& a, cudaStream_t s) {
-    k_om_perm<T, PLC, false><<<grid_perm(a), 256, smem_perm, s>>>(a);
+    launch_pdl<true>(k_om_perm<T, PLC, false, true>, grid_perm(a), 256, smem_perm, s, a);
   }
   static const AdjKernels* get() {
     if constexpr (FX) {
