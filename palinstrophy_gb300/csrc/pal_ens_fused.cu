@@ -131,30 +131,34 @@ struct FusedOf {
 };
 
 // The 96-member configuration's sizes: N = 256, 384, 512 (M = 384, 576, 768).
-// One block size for all bodies means one register budget (the largest body's):
-// the light plans are chosen (the 6.6.16 row plan at N=384 needs ~60 registers
-// where the 24.24 plan needs 128).
-using P384 = Plan<384, 16, 24>;
-using P576 = Plan<576, 24, 24>;
-using P576b = Plan<576, 6, 6, 16>;
-using P768 = Plan<768, 32, 24>;
-using P768b = Plan<768, 16, 2, 24>;
+// One block size for all bodies means one register budget (the largest body's),
+// so the plans are those with the smallest radices, which also give a short
+// tile the most threads to hide its loads and barriers with.  us per CNAB2 step
+// of the 96 members, GB300: 286 with these plans, row tiles of 192 threads and
+// column passes of 64; 357 with 16.24 / 6.6.16 / 16.2.24 rows on 128 threads
+// and 16.24 / 24.24 / 32.24 columns on 64 (the rows give 46 of it, the columns
+// 24); 418 for per-size launches of each size's own candidates.  Row tiles of 4
+// lines on 256 and 384 threads: 317 and 377, of 8 lines on 384: 309 (fewer
+// tiles in flight); columns on 48 threads 303, on 96 or 128 346 (64: 333, all
+// three with the old rows); rows without TMA 298.  Fewer registers (minimum
+// blocks per SM) for either pass: 286.  The passes are bound by issue and
+// latency, not by memory: stepping quarters of the members one after the other,
+// whose state then stays in L2, took 320, the gain lost to the launches' tails.
+using P384 = Plan<384, 6, 8, 8>;
+using P576 = Plan<576, 6, 8, 12>;
+using P768 = Plan<768, 8, 8, 12>;
 using S256 = FusedSize<Rec<P384>, 4, 14, Rec<P384>, 2>;
-using S384 = FusedSize<Rec<P576b>, 2, 14, Rec<P576>, 2>;
-using S512 = FusedSize<Rec<P768b>, 4, 14, Rec<P768>, 2>;
-// Row tiles of 128 threads, column passes of 64: measured 2620 ensemble steps/s
-// for the 96-member configuration, against 2557 with the plain radix-16.24
-// column at N=256, 2153 with 128-thread column blocks, and 2505 for per-size
-// launches of candidates re-tuned on each group's batched shape.
-using F3 = FusedOf<128, 64, S256, S384, S512>;
+using S384 = FusedSize<Rec<P576>, 4, 14, Rec<P576>, 2>;
+using S512 = FusedSize<Rec<P768>, 4, 14, Rec<P768>, 2>;
+using F3 = FusedOf<192, 64, S256, S384, S512>;
 
 const FusedSet kSet3 = {3,
                         {256, 384, 512},
-                        {"16.24r V4x128 tma-in tma-out", "6.6.16r V2x128 tma-in tma-out",
-                         "16.2.24r V4x128 tma-in tma-out"},
-                        {"16.24r x128 hoist", "24.24r x128 hoist", "32.24r x128 hoist"},
-                        {4, 2, 4},
-                        128,
+                        {"6.8.8r V4x192 tma-in tma-out", "6.8.12r V4x192 tma-in tma-out",
+                         "8.8.12r V4x192 tma-in tma-out"},
+                        {"6.8.8r x128 hoist", "6.8.12r x192 hoist", "8.8.12r x192 hoist"},
+                        {4, 4, 4},
+                        192,
                         F3::smem_row,
                         F3::smem_col,
                         F3::smem_perm,

@@ -31,7 +31,8 @@ const RowKernels r384[] = {RowOf<float, P576, 4, 256>::make("24.24 V4x256"),
                            RowOf<float, Rec<P576>, 4, 256, 15>::make("24.24r V4x256 tma-in tma-out l2pf"),
                            RowOf<float, Rec<P576b>, 4, 192, 15>::make("6.6.16r V4x192 tma-in tma-out l2pf"),
                            RowOf<float, Rec<P576b>, 4, 192, 14>::make("6.6.16r V4x192 tma-in tma-out"),
-                           RowOf<float, Rec<P576b>, 2, 128, 14>::make("6.6.16r V2x128 tma-in tma-out")};
+                           RowOf<float, Rec<P576b>, 2, 128, 14>::make("6.6.16r V2x128 tma-in tma-out"),
+                           RowOf<float, Rec<P576c>, 4, 192, 14>::make("6.8.12r V4x192 tma-in tma-out")};
 const ColKernels c384[] = {ColOf<float, P576, 128>::make("24.24 x128"), ColOf<float, P576b, 128>::make("6.6.16 x128"),
                            ColOf<float, Rec<P576>, 128, 2>::make("24.24r x128 hoist"),
                            ColOf<float, Rec<P576c>, 192, 2>::make("6.8.12r x192 hoist")};
@@ -44,7 +45,8 @@ const RowKernels r512[] = {RowOf<float, P768, 4, 256>::make("32.24 V4x256"),
                            RowOf<float, Rec<P768b>, 4, 256, 15>::make("16.2.24r V4x256 tma-in tma-out l2pf"),
                            RowOf<float, Rec<P768>, 4, 128, 15>::make("32.24r V4x128 tma-in tma-out l2pf"),
                            RowOf<float, Rec<P768b>, 4, 128, 14>::make("16.2.24r V4x128 tma-in tma-out"),
-                           RowOf<float, Rec<P768c>, 2, 192, 2>::make("8.8.12r V2x192 paired")};
+                           RowOf<float, Rec<P768c>, 2, 192, 2>::make("8.8.12r V2x192 paired"),
+                           RowOf<float, Rec<P768c>, 4, 192, 14>::make("8.8.12r V4x192 tma-in tma-out")};
 const ColKernels c512[] = {ColOf<float, P768, 128>::make("32.24 x128"), ColOf<float, P768b, 128>::make("16.2.24 x128"),
                            ColOf<float, P768, 256>::make("32.24 x256"),
                            ColOf<float, Rec<P768>, 128, 2>::make("32.24r x128 hoist"),
