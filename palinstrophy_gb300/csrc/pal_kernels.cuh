@@ -1675,9 +1675,12 @@ __global__ void __launch_bounds__(NT, MINB) k_col_tma(StepArgs a0, const __grid_
 // apart: without the pad slot after every STEP entries a warp's shared-memory
 // accesses all fell into one bank.  One array per block (grid.z) halves the
 // tile, so three to six blocks share an SM where one or two did.  F_NO_FM_IN:
-// fnm1 is left out (the first RK3 stage does not read it).  N=8192 FP32: 1030 /
-// 880 us before (to / from the butterfly-major order, both arrays), now 174 us
-// for om alone / 345 us (3.1 TB/s); N=4096 143 / 99 us before, now 32 / 56 us.
+// fnm1 is left out (the first RK3 stage does not read it).  The natural side
+// moves 16 bytes a thread and the butterfly side loads all of a butterfly before
+// it stores any: with 8 bytes and loads mixed with shared-memory stores too few
+// bytes were in flight.  N=8192 FP32, to / from the butterfly-major order: 1030 /
+// 880 us at first (both arrays), 174 (om alone) / 345 us with the padded tile
+// alone, now 118 / 178 us (4.5 / 6.0 TB/s); N=4096 143 / 99, 32 / 56, 24 / 35 us.
 template <typename T, class PL>
 struct PermTile {
   static constexpr int N = 2 * PL::M / 3;
@@ -1695,8 +1698,19 @@ __device__ __forceinline__ void om_perm_column(cplx<T>* sm, cplx<T>* __restrict_
   constexpr int RP = PL::RP, FSTEP = PL::FSTEP;
   constexpr bool BAND_CT = (RP % 3 == 0) && ((RP / 3) % 2 == 0);  // the pad is the middle third of the j
   if constexpr (TO_PERM) {
-#pragma unroll 4
-    for (int z = tid; z < N; z += NT) sm[PT::slot(z)] = nat[z];
+    // 16 bytes a load, eight in flight: a column starts on a multiple of 16 bytes
+    // (N is a multiple of 4) and STEP is even, so both of a pair lie in one group
+    if constexpr (sizeof(C) == 8 && PT::STEP % 2 == 0) {
+#pragma unroll 8
+      for (int z = 2 * tid; z < N; z += 2 * NT) {
+        const float4 p = *reinterpret_cast<const float4*>(nat + z);
+        sm[PT::slot(z)] = C{p.x, p.y};
+        sm[PT::slot(z) + 1] = C{p.z, p.w};
+      }
+    } else {
+#pragma unroll 8
+      for (int z = tid; z < N; z += NT) sm[PT::slot(z)] = nat[z];
+    }
     __syncthreads();
   }
   // a thread takes one butterfly's entries, every G-th of them where there are
@@ -1705,24 +1719,46 @@ __device__ __forceinline__ void om_perm_column(cplx<T>* sm, cplx<T>* __restrict_
   for (int w = tid; w < G * FSTEP; w += NT) {
     const int b = w % FSTEP, j0 = w / FSTEP;
     const int fb = PL::freq(b * RP);
-#pragma unroll
-    for (int jj = 0; jj < RP; jj += G) {
-      const int j = G == 1 ? jj : jj + j0;
-      if (RP % G != 0 && j >= RP) continue;
-      if (BAND_CT && j >= RP / 3 && j < 2 * (RP / 3)) continue;
+    // slot of entry j in the tile, < 0 in the pad
+    auto place = [&](int j) {
+      if (RP % G != 0 && j >= RP) return -1;
+      if (BAND_CT && j >= RP / 3 && j < 2 * (RP / 3)) return -1;
       const int f = fb + j * FSTEP;
-      if (!BAND_CT && f >= Nh && f < N) continue;
-      const int z = f < Nh ? f : f - Nh;
-      if constexpr (TO_PERM)
-        perm[j * FSTEP + b] = sm[PT::slot(z)];
-      else
-        sm[PT::slot(z)] = perm[j * FSTEP + b];
+      if (!BAND_CT && f >= Nh && f < N) return -1;
+      return PT::slot(f < Nh ? f : f - Nh);
+    };
+    if constexpr (TO_PERM) {
+#pragma unroll
+      for (int jj = 0; jj < RP; jj += G) {
+        const int j = G == 1 ? jj : jj + j0, at = place(j);
+        if (at >= 0) perm[j * FSTEP + b] = sm[at];
+      }
+    } else {
+      C x[(RP + G - 1) / G];  // every load of the butterfly in flight at once
+#pragma unroll
+      for (int jj = 0; jj < RP; jj += G) {
+        const int j = G == 1 ? jj : jj + j0;
+        if (place(j) >= 0) x[jj / G] = perm[j * FSTEP + b];
+      }
+#pragma unroll
+      for (int jj = 0; jj < RP; jj += G) {
+        const int at = place(G == 1 ? jj : jj + j0);
+        if (at >= 0) sm[at] = x[jj / G];
+      }
     }
   }
   __syncthreads();
   if constexpr (!TO_PERM) {
-#pragma unroll 4
-    for (int z = tid; z < N; z += NT) nat[z] = sm[PT::slot(z)];
+    if constexpr (sizeof(C) == 8 && PT::STEP % 2 == 0) {
+#pragma unroll 8
+      for (int z = 2 * tid; z < N; z += 2 * NT) {
+        const C p = sm[PT::slot(z)], q = sm[PT::slot(z) + 1];
+        *reinterpret_cast<float4*>(nat + z) = float4{float(p.x), float(p.y), float(q.x), float(q.y)};
+      }
+    } else {
+#pragma unroll 8
+      for (int z = tid; z < N; z += NT) nat[z] = sm[PT::slot(z)];
+    }
   }
 }
 template <typename T, class PL, bool TO_PERM, int NT>
