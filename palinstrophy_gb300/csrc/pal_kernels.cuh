@@ -980,11 +980,9 @@ __global__ void __launch_bounds__(NT, (PF & 16) ? row_tiles_per_sm<T, PL, V>() :
   row_body<T, PL, V, NT, PF>(a0, maps, hw_blk());
 }
 
-// The diagnostic sum of u^2 + v^2 of one thread: the squares of four points run
-// into one FP64 chain of fused multiply-adds, and the chain's value is added to
-// the compensated sum.  The diagnostic k_phys is bound by the FP64 pipe: 5 FP64
-// instructions a point (conversions included) where a TwoSum per point took 11;
-// N=2048 FP32 295 us before, 173 now.
+// The diagnostic sum of u^2 + v^2 of one thread in FP64: the squares of four
+// points run into one chain of fused multiply-adds, and the chain's value is
+// added to the compensated sum.
 struct SquareSum {
   double s = 0.0;
   int n = 0;
@@ -999,8 +997,48 @@ struct SquareSum {
   }
 };
 
+// u^2 + v^2 of G FP32 points added to a compensated sum: every square is exact
+// in integers (24-bit mantissas) at the exponent of the group's largest value,
+// so the group's sum is off by the bits shifted out alone (below 2^-54 of it)
+// and takes 6 instructions of the FP64 pipe, which gives a warp one in 64
+// cycles; fused multiply-adds on the widened values took 3 a point.  With it and
+// k_phys's paired first pass the diagnostic k_phys of N=2048 takes 72 us where
+// it took 173 (and 295 with a TwoSum per point).
+template <int G>
+__device__ __forceinline__ void add_squares(const float2 (&x)[G], double& acc, double& comp) {
+  static_assert(G <= 8, "2 G squares below 2^58 fit in 64 bits");
+  constexpr unsigned MAG = 0x7fffffffu, FRAC = 0x7fffffu;
+  unsigned top = 0;
+#pragma unroll
+  for (int i = 0; i < G; ++i)
+    top = max(top, max(__float_as_uint(x[i].x) & MAG, __float_as_uint(x[i].y) & MAG));
+  if (top > MAG - (FRAC + 1)) {  // an infinity or NaN
+    double s = 0.0;
+#pragma unroll
+    for (int i = 0; i < G; ++i) s = fma(double(x[i].x), double(x[i].x), fma(double(x[i].y), double(x[i].y), s));
+    csum_add_pos(acc, comp, s);
+    return;
+  }
+  const int E = max((int)(top >> 23), 1);  // subnormals have exponent 1 and no leading bit
+  unsigned long long q = 0;
+  auto add = [&](float f) {
+    const unsigned b = __float_as_uint(f) & MAG, e = b >> 23;
+    const unsigned m = ((b & FRAC) | (e != 0 ? FRAC + 1 : 0u)) << 5;
+    q += ((unsigned long long)m * m) >> min(2 * (E - max((int)e, 1)), 63);
+  };
+#pragma unroll
+  for (int i = 0; i < G; ++i) {
+    add(x[i].x);
+    add(x[i].y);
+  }
+  // q 2^-10 (2^(E - 150))^2
+  csum_add_pos(acc, comp, (double)q * __hiloint2double((1023 + 2 * (E - 150) - 10) << 20, 0));
+}
+
 // k_phys: U-state rows -> physical u, v (statistics, optional plane store).  A
 // block takes every bk.nx-th of the M / V tiles and reduces its statistics once.
+// The first pass is the row pass's paired one: it builds both halves of the
+// Hermitian pack from one read of the planes.
 // Dynamic shared memory: the tile, at least 2 NT doubles (finish_stats).
 template <typename T, class PL, int V, int NT>
 __device__ __forceinline__ void phys_body(const StepArgs& a0, const Blk bk) {
@@ -1016,31 +1054,42 @@ __device__ __forceinline__ void phys_body(const StepArgs& a0, const Blk bk) {
   T* __restrict__ ph = static_cast<T*>(a.phys);
   const bool store = (a.flags & F_PHYS) != 0;
   const bool diag = (a.flags & F_DIAG) != 0;
-  SquareSum quad;
+  constexpr int G = 8;  // points read at once
   for (int tile = bk.x; tile < M / V; tile += bk.nx) {
     const int z0 = tile * V;
-    row_first_pass<T, PL, V, NT>(a, sm, z0, tid);
+    if constexpr ((M / PL::R[0]) % 2 == 0 && PL::R[0] % 2 == 0)
+      row_first_pass_paired<T, PL, V, NT>(a, sm, z0, tid);
+    else
+      row_first_pass<T, PL, V, NT>(a, sm, z0, tid);
     dif_range<T, PL, V, NT, +1, 1, PL::NP>(sm, tw, tid);
-    for (int w = tid; w < V * M; w += NT) {
-      const int v = w % V;
-      const int pos = w / V;
-      const C val = sm[PL::phys(pos) * V + v];
-      mx = fmax(mx, fabs(val.x) + fabs(val.y));
+    for (int w0 = tid; w0 < V * M; w0 += G * NT) {
+      C x[G];
+#pragma unroll
+      for (int i = 0; i < G; ++i) {
+        const int w = w0 + i * NT;
+        x[i] = w < V * M ? sm[PL::phys(w / V) * V + w % V] : C{T(0), T(0)};
+      }
+#pragma unroll
+      for (int i = 0; i < G; ++i) mx = fmax(mx, fabs(x[i].x) + fabs(x[i].y));
       if (diag) {
-        quad.add(widen(val.x), widen(val.y), acc, comp);
+        add_squares(x, acc, comp);
       } else {
-        accp = fma(val.x, val.x, fma(val.y, val.y, accp));  // finiteness check only
+#pragma unroll
+        for (int i = 0; i < G; ++i) accp = fma(x[i].x, x[i].x, fma(x[i].y, x[i].y, accp));  // finiteness check only
       }
       if (store) {
-        const int n = PL::freq(pos);
-        ph[(size_t)(z0 + v) * M + n] = val.x;
-        ph[(size_t)M * M + (size_t)(z0 + v) * M + n] = val.y;
+#pragma unroll
+        for (int i = 0; i < G; ++i) {
+          const int w = w0 + i * NT, n = PL::freq(w / V), v = w % V;
+          if (w >= V * M) continue;
+          ph[(size_t)(z0 + v) * M + n] = x[i].x;
+          ph[(size_t)M * M + (size_t)(z0 + v) * M + n] = x[i].y;
+        }
       }
     }
     __syncthreads();  // the tile is free
   }
   if (diag) {
-    quad.flush(acc, comp);
     finish_stats<NT, true>(a, double(mx), acc, comp, M, tid, bk, reinterpret_cast<double*>(smraw));
   } else {
     finish_stats<NT, false>(a, double(mx), double(accp), 0.0, M, tid, bk);

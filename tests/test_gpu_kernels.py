@@ -216,3 +216,27 @@ def test_spectral_sums(N, prec):
     for key, ref in (("E", E), ("L", 2.0 * math.pi * S / E), ("Z", math.fsum(p.ravel()) - p[0, 0]),
                      ("P", math.fsum((k2 * p).ravel()))):
         assert abs(d[key] - ref) <= 16 * np.finfo(np.float64).eps * ref, key
+
+
+@pytest.mark.parametrize("scale", [1e-42, 1e-30, 1.0, 1e16])
+@pytest.mark.parametrize("N", [32, 384, 1024, 2048])
+def test_mean_square_velocity(N, scale):
+    """The diagnostic sum of u^2 + v^2 of an FP32 field against the exactly
+    rounded sum of its squares (exact in FP64): the sum is off by a rounding per
+    group and by its shifted-out bits, U by half of that, its square root and
+    quotient.  Scales: subnormal and small velocities, ordinary ones, large ones."""
+    import math
+
+    from palinstrophy_gb300.turbo_simulator import Field
+
+    om = (_spectrum(N, "k-1") * scale).astype(np.complex64)
+    F = Field(N, "fp32", 1e3, 0.3)
+    F.set_state(om)
+    F.set_scalars(dt=1e-3)
+    U = F.diagnostics()["U"]
+    F.step2a()
+    u, v = (np.asarray(F.ur(i), np.float64).ravel() for i in (0, 1))
+    F.close()
+    ref = math.sqrt(math.fsum(u * u + v * v) / u.size)
+    assert ref > 0.0
+    assert abs(U - ref) <= 4 * np.finfo(np.float64).eps * ref
