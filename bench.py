@@ -11,7 +11,7 @@ Printed JSON line (rank 0):
   value      FP32-form steps/s, whole job (N ranks x replicas), device-timed with
              CUDA events on the handle's stream, state resident in HBM; the
              state (0.67 GB) is larger than L2, so no flush is needed.
-  fp64       the plain FP64 path on the same GPU and workload
+  fp64       the FP64 form on the same GPU and workload
   e2e        the same metric through the C ABI from pinned host buffers: upload
              of the initial om2 + velocity band, initial NEXTDT, K steps with the
              run_dns NEXTDT cadence (host reads CFLM/dt at each update), and the
@@ -30,8 +30,8 @@ worker count min(8, cores), for a bounded number of steps; it imports nothing
 from palinstrophy_gb300.
 
 rel_l2_fp32_vs_oracle_100_steps: the FP64 oracle runs 100 steps from the same
-start in a spawned process while the GPU legs run; the FP32 form and the FP64
-plain path then replay its dt / cn sequence and are compared with it.
+start in a spawned process while the GPU legs run; the FP32 and the FP64
+form then replay its dt / cn sequence and are compared with it.
 """
 from __future__ import annotations
 
@@ -157,55 +157,30 @@ def _limiter(kernel, prec):
             f"FP32 FMA pipe {fma} (profiles/{kernel}_{prec}_N{N_GRID}.md)")
 
 
-def _fp64_counts(kernel, cand):
-    """(FP64 flops, FP64 pipe instructions) per launch of the FP64 plain path's
-    kernel candidate `cand` at N=4096, from the committed ncu summary: flops =
-    2 DFMA + DADD + DMUL thread instructions, pipe instructions = their sum."""
-    path = os.path.join(ROOT, "profiles", f"kernels_fp64_N{N_GRID}.md")
-    out = {}
-    try:
-        with open(path) as f:
-            for line in f:
-                for key in ("flops", "pipe_inst"):
-                    tag = f"fp64_{key}_per_launch_{kernel}[{cand}]:"
-                    if line.strip().startswith(tag):
-                        out[key] = float(line.split(":", 1)[1].split()[0])
-    except OSError:
-        pass
-    return out.get("flops"), out.get("pipe_inst")
-
-
 def _fp64_roofline(om2, uc, visc):
-    """The FP64 plain path against its own ceiling: counted FP64 flops per k_row /
-    k_col launch (ncu instruction counts, profiles/) over the launch times measured
-    here, against the FP64 FMA throughput measured here (pal_fp64_peak); and the
-    same launches' algorithmic bytes against the measured HBM bandwidth."""
+    """The FP64 form's two kernels against the measured HBM bandwidth.  Their
+    transforms run in 64-bit integers (fixed point) and the spectral update in
+    FP64, so what bounds them is the issue of 64-bit integer multiply-adds and,
+    in the column pass, the FP64 pipe, whose measured FMA peak is given too
+    (pal_fp64_peak)."""
     from palinstrophy_gb300 import _lib as L
     F = _field("fp64", om2, uc, visc)
     ms_row, ms_col, _ = F.profile_kernels(METHOD, 2)
     desc = F.variant()["desc"]
     F.close()
-    peak, peak_ms = L.fp64_peak()
-    hbm, _ = _peaks()
+    fp64_peak, peak_ms = L.fp64_peak()
+    hbm, hbm_kind = _peaks()
     n2 = float(N_GRID) * N_GRID
-    out = {"bound": "fp64", "unit": "TFLOP/s", "peak": peak,
-           "peak_kind": f"measured: FP64 FMA-chain microbenchmark (pal_fp64_peak, {peak_ms:.1f} ms launch)",
-           "kernels": desc}
-    cands = {"k_row": desc.split("row[")[1].split("]")[0], "k_col": desc.split("col[")[1].split("]")[0]}
+    out = {"bound": "integer and FP64 issue", "unit": "GB/s", "peak": hbm, "peak_kind": hbm_kind, "kernels": desc,
+           "fp64_peak_tflops": fp64_peak,
+           "fp64_peak_kind": f"measured: FP64 FMA-chain microbenchmark (pal_fp64_peak, {peak_ms:.1f} ms launch)"}
     for name, ms, nbytes in (("k_row", ms_row, 6.0 * n2 * 8), ("k_col", ms_col, (25.0 / 3.0) * n2 * 8)):
-        fl, inst = _fp64_counts(name, cands[name])
-        ach = fl / (ms / 1000.0) / 1e12 if fl else None
-        # the FP64 pipe takes one instruction per slot whether DFMA (2 flops) or
-        # DADD / DMUL (1 flop): the pipe fraction is the FFT's real ceiling
-        pipe = inst / (ms / 1000.0) / (peak * 1e12 / 2.0) if inst else None
-        out[name] = {"ms": ms, "candidate": cands[name], "flops_per_launch": fl, "achieved": ach,
-                     "frac": ach / peak if ach else None, "pipe_inst_per_launch": inst, "pipe_frac": pipe,
-                     "hbm_GBps": nbytes / (ms / 1000.0) / 1e9, "hbm_frac": nbytes / (ms / 1000.0) / 1e9 / hbm}
+        gbs = nbytes / (ms / 1000.0) / 1e9
+        out[name] = {"ms": ms, "algorithmic_bytes": nbytes, "hbm_GBps": gbs, "hbm_frac": gbs / hbm}
     dom = "k_row" if ms_row >= ms_col else "k_col"
     out["kernel"] = dom
-    out["achieved"] = out[dom]["achieved"]
-    out["frac"] = out[dom]["frac"]
-    out["pipe_frac"] = out[dom]["pipe_frac"]
+    out["achieved"] = out[dom]["hbm_GBps"]
+    out["frac"] = out[dom]["hbm_frac"]
     return out
 
 
@@ -432,7 +407,7 @@ def _rel_l2(a, b):
 
 def _precision_form(steps=2000, update=100):
     """N=1024, labelled k^4 exp(-2 (k/15)^2) unit-energy start (seed 4895), Re=1e4,
-    LS-IMEX-RK3 at CFL 0.1: the FP32 form and the FP64 plain path from the identical
+    LS-IMEX-RK3 at CFL 0.1: the FP32 and the FP64 form from the identical
     start, each with its own adaptive dt; steps/s of each and their agreement."""
     import numpy as np
     import torch
@@ -485,7 +460,7 @@ def _embed_spectrum(om2, N):
 def _large_single_field(om2, uc, visc, steps_8192=30, drift_steps=500, every=100):
     """N=8192 FP32 (KM3 K0=15 seed 4895, Re=1e5, LS-IMEX-RK3, CFL 0.1): steps/s and
     per-kernel rates; the energy / enstrophy history of the N=4096 FP32 form
-    against the FP64 plain run over 500 steps from the identical start; and
+    against the FP64 run over 500 steps from the identical start; and
     500 N=8192 FP32 steps of the same flow against that FP64 run."""
     import numpy as np
     import torch
@@ -657,7 +632,7 @@ class _OracleRun:
 
 
 def _vs_oracle(om2, uc, visc, oracle):
-    """rel-L2 of om2 after the oracle's steps, FP32 form and FP64 plain path from
+    """rel-L2 of om2 after the oracle's steps, FP32 and FP64 form from
     the identical start, the oracle's dt / cn sequence replayed into the GPU run."""
     from palinstrophy_gb300.turbo_simulator import Field
     o_om2, log, secs, threads = oracle.result()
@@ -744,7 +719,7 @@ def run_gb300(args):
     F = _field("fp32", om2, uc, visc)
     ms32, clocks = _timed_steps(F, args.steps, args.warmup, sampler_index=local)
     F.close()
-    # FP64 plain path
+    # FP64 form
     k64 = max(3, args.steps // 40)
     F = _field("fp64", om2, uc, visc)
     ms64, _ = _timed_steps(F, k64, max(3, args.warmup // 10))
@@ -758,7 +733,7 @@ def run_gb300(args):
     if rank != 0:
         return
 
-    # accuracy: FP32 form vs FP64 plain after 100 steps from the identical start
+    # accuracy: FP32 form vs FP64 form after 100 steps from the identical start
     A = _field("fp32", om2, uc, visc)
     B = _field("fp64", om2, uc, visc)
     A.step(METHOD, 100, update=UPDATE, final_update=True)

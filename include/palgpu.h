@@ -161,7 +161,7 @@ int pal_synchronize(pal_handle* h);
 int pal_profile_kernels(pal_handle* h, int method, int nsteps, double* ms_row, double* ms_col, int* launches);
 /* FP64 FMA throughput of the current GPU in TFLOP/s (best of 5 timed launches of
  * an FMA-chain kernel filling every SM, CUDA events; *ms = that launch's time):
- * the ceiling of the FP64 plain path, whose kernels are bound by the FP64 pipe.
+ * the ceiling of what the FP64 form still does in FP64 (the spectral update).
  * Measurement support; no counterpart in the reference. */
 int pal_fp64_peak(double* tflops, double* ms);
 /* Kernel candidates: for each N the library compiles several row-pass and

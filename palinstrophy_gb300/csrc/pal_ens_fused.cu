@@ -137,7 +137,7 @@ struct FusedOf {
 // of the 96 members, GB300: 286 with these plans, row tiles of 192 threads and
 // column passes of 64; 357 with 16.24 / 6.6.16 / 16.2.24 rows on 128 threads
 // and 16.24 / 24.24 / 32.24 columns on 64 (the rows give 46 of it, the columns
-// 24); 418 for per-size launches of each size's own candidates.  Row tiles of 4
+// 24); 418 for per-size launches of the single fields' candidates, 345 re-tuned.  Row tiles of 4
 // lines on 256 and 384 threads: 317 and 377, of 8 lines on 384: 309 (fewer
 // tiles in flight); columns on 48 threads 303, on 96 or 128 346 (64: 333, all
 // three with the old rows); rows without TMA 298.  Fewer registers (minimum

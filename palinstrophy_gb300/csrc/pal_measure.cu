@@ -1,5 +1,5 @@
 // Measurement support: the FP64 FMA throughput of the GPU, the ceiling of the
-// FP64 plain path (its kernels are bound by the FP64 pipe, not by HBM).  No
+// spectral update of the FP64 form (its transforms are integers).  No
 // counterpart in the reference.
 //
 // k_fp64_fma: every thread runs kChains independent FMA chains x <- x a + b for
