@@ -20,6 +20,7 @@
 #include <math.h>
 
 #include "pal_fft.cuh"
+#include "pal_sums.cuh"
 
 namespace pal {
 
@@ -240,16 +241,6 @@ __device__ __forceinline__ void block_maxsum(double& m, double& s, double* red /
   __syncthreads();
 }
 
-// Compensated FP64 summation: s + c carries the running sum, c the exact
-// rounding errors of the additions into s (TwoSum, which needs no ordering of
-// the operands' magnitudes).
-__device__ __forceinline__ void csum_add(double& s, double& c, double x) {
-  const double t = s + x;
-  const double bp = t - s;
-  c += (s - (t - bp)) + (x - bp);
-  s = t;
-}
-
 // A float in FP64 without the FP64 pipe: its bits, rebiased (the pipe's own
 // conversion for zeros, subnormals, infinities and NaN).
 __device__ __forceinline__ double widen(float x) {
@@ -258,16 +249,6 @@ __device__ __forceinline__ double widen(float x) {
   return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + (896u << 20))), (int)(b << 29));
 }
 __device__ __forceinline__ double widen(double x) { return x; }
-
-// csum_add for s, x >= 0 (no NaN ordering is needed: a NaN stays one): the
-// larger operand is found on the bit patterns, and then Fast2Sum's four FP64
-// instructions do what TwoSum needs seven for.
-__device__ __forceinline__ void csum_add_pos(double& s, double& c, double x) {
-  const long long is = __double_as_longlong(s), ix = __double_as_longlong(x);
-  const double hi = __longlong_as_double(max(is, ix)), lo = __longlong_as_double(min(is, ix));
-  s = hi + lo;
-  c += lo - (s - hi);
-}
 
 // Block-wide compensated sum of K pairs (s, c), in red (2 K NT doubles): the
 // pairs cross shared memory and warp q alone adds those of sum q, the s parts
@@ -996,44 +977,6 @@ struct SquareSum {
     n = 0;
   }
 };
-
-// u^2 + v^2 of G FP32 points added to a compensated sum: every square is exact
-// in integers (24-bit mantissas) at the exponent of the group's largest value,
-// so the group's sum is off by the bits shifted out alone (below 2^-54 of it)
-// and takes 6 instructions of the FP64 pipe, which gives a warp one in 64
-// cycles; fused multiply-adds on the widened values took 3 a point.  With it and
-// k_phys's paired first pass the diagnostic k_phys of N=2048 takes 72 us where
-// it took 173 (and 295 with a TwoSum per point).
-template <int G>
-__device__ __forceinline__ void add_squares(const float2 (&x)[G], double& acc, double& comp) {
-  static_assert(G <= 8, "2 G squares below 2^58 fit in 64 bits");
-  constexpr unsigned MAG = 0x7fffffffu, FRAC = 0x7fffffu;
-  unsigned top = 0;
-#pragma unroll
-  for (int i = 0; i < G; ++i)
-    top = max(top, max(__float_as_uint(x[i].x) & MAG, __float_as_uint(x[i].y) & MAG));
-  if (top > MAG - (FRAC + 1)) {  // an infinity or NaN
-    double s = 0.0;
-#pragma unroll
-    for (int i = 0; i < G; ++i) s = fma(double(x[i].x), double(x[i].x), fma(double(x[i].y), double(x[i].y), s));
-    csum_add_pos(acc, comp, s);
-    return;
-  }
-  const int E = max((int)(top >> 23), 1);  // subnormals have exponent 1 and no leading bit
-  unsigned long long q = 0;
-  auto add = [&](float f) {
-    const unsigned b = __float_as_uint(f) & MAG, e = b >> 23;
-    const unsigned m = ((b & FRAC) | (e != 0 ? FRAC + 1 : 0u)) << 5;
-    q += ((unsigned long long)m * m) >> min(2 * (E - max((int)e, 1)), 63);
-  };
-#pragma unroll
-  for (int i = 0; i < G; ++i) {
-    add(x[i].x);
-    add(x[i].y);
-  }
-  // q 2^-10 (2^(E - 150))^2
-  csum_add_pos(acc, comp, (double)q * __hiloint2double((1023 + 2 * (E - 150) - 10) << 20, 0));
-}
 
 // k_phys: U-state rows -> physical u, v (statistics, optional plane store).  A
 // block takes every bk.nx-th of the M / V tiles and reduces its statistics once.
