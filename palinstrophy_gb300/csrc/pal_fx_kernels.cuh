@@ -352,7 +352,6 @@ __global__ void __launch_bounds__(NT) k_phys_fx(StepArgs a0) {
   double* __restrict__ ph = static_cast<double*>(a.phys);
   const bool store = (a.flags & F_PHYS) != 0;
   const bool diag = (a.flags & F_DIAG) != 0;
-  SquareSum quad;
   for (int tile = bk.x; tile < M / V; tile += bk.nx) {
     const int z0 = tile * V;
     FxScale sc;
@@ -365,7 +364,7 @@ __global__ void __launch_bounds__(NT) k_phys_fx(StepArgs a0) {
       const double x = fx_value(q.x, sc), y = fx_value(q.y, sc);
       top = max(top, fx_speed(q));
       if (diag)
-        quad.add(x, y, acc, comp);
+        add_point(x, y, acc, comp);
       else
         acc = fma(x, x, fma(y, y, acc));  // finiteness check only
       if (store) {
@@ -378,7 +377,6 @@ __global__ void __launch_bounds__(NT) k_phys_fx(StepArgs a0) {
     __syncthreads();  // the tile and its words are free
   }
   if (diag) {
-    quad.flush(acc, comp);
     finish_stats<NT, true>(a, mx, acc, comp, M, tid, bk, reinterpret_cast<double*>(smraw));
   } else {
     finish_stats<NT, false>(a, mx, acc, 0.0, M, tid, bk);

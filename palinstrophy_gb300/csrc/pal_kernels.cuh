@@ -961,23 +961,6 @@ __global__ void __launch_bounds__(NT, (PF & 16) ? row_tiles_per_sm<T, PL, V>() :
   row_body<T, PL, V, NT, PF>(a0, maps, hw_blk());
 }
 
-// The diagnostic sum of u^2 + v^2 of one thread in FP64: the squares of four
-// points run into one chain of fused multiply-adds, and the chain's value is
-// added to the compensated sum.
-struct SquareSum {
-  double s = 0.0;
-  int n = 0;
-  __device__ __forceinline__ void add(double u, double v, double& acc, double& comp) {
-    s = fma(u, u, fma(v, v, s));
-    if (++n == 4) flush(acc, comp);
-  }
-  __device__ __forceinline__ void flush(double& acc, double& comp) {
-    csum_add_pos(acc, comp, s);
-    s = 0.0;
-    n = 0;
-  }
-};
-
 // k_phys: U-state rows -> physical u, v (statistics, optional plane store).  A
 // block takes every bk.nx-th of the M / V tiles and reduces its statistics once.
 // The first pass is the row pass's paired one: it builds both halves of the

@@ -2,6 +2,7 @@
 // run the same arithmetic.
 #pragma once
 #include <cuda_runtime.h>
+#include <math.h>
 #include <string.h>
 
 namespace pal {
@@ -32,6 +33,11 @@ __host__ __device__ __forceinline__ void csum_add_pos(double& s, double& c, doub
   const double hi = bits_as<double>(is > ix ? is : ix), lo = bits_as<double>(is > ix ? ix : is);
   s = hi + lo;
   c += lo - (s - hi);
+}
+
+// u^2 + v^2 of an FP64 point added to a compensated sum.
+__host__ __device__ __forceinline__ void add_point(double u, double v, double& acc, double& comp) {
+  csum_add_pos(acc, comp, fma(u, u, v * v));
 }
 
 // u 2^e in FP64 without the FP64 pipe, rounded to nearest (halves up); the

@@ -53,3 +53,16 @@ def test_squares_of_float_points_are_summed_beyond_double(sums):
     for g, s in zip(gs, got):
         exact = sum(Fraction(float(v)) ** 2 for v in g)
         assert abs(s - exact) <= exact / 2 ** 56, g
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 48])
+def test_squares_of_double_points_are_compensated_one_by_one(sums, n):
+    """n equal points add up to n times the rounded point: a compensated sum's
+    own error is of the order n 2^-106, a plain chain of four has roundings of
+    2^-53 in it."""
+    rng = np.random.default_rng(n)
+    uv = rng.standard_normal((300, 2)) * 2.0 ** rng.integers(-20, 20, (300, 1))
+    got = sums([f"p {n} " + " ".join(f"{b:x}" for b in p.view(np.uint64)) for p in uv])
+    for (u, v), s in zip(uv, got):
+        point = Fraction(float(Fraction(u) ** 2 + Fraction(float(v * v))))
+        assert abs(s - n * point) <= n * point / 2 ** 100
