@@ -1842,13 +1842,23 @@ __device__ __forceinline__ double int_rsqrt(double x, int ix) {
   return fma(y, e * fma(e, 0.375, 0.5), y);
 }
 
+// p / K2 for ik = r^2, r the reciprocal root of K2: the product, up to 4 units
+// of 2^-53 off, is corrected by its remainder, so that one rounding is left as
+// after a division.
+__device__ __forceinline__ double over_k2(double p, double K2, double ik) {
+  const double e = p * ik;
+  const double f = fma(ik, fma(-K2, e, p), e);
+  return finite_bits(e) ? f : e;
+}
+
 // Spectral sums over om [kx][z]: E = sum w |om|^2/K2, Lsum = sum w |om|^2/K2^1.5,
 // Z = sum w |om|^2 (minus the (0,0) mode), P = sum w K2 |om|^2, with the
 // rfft weights w = [1, 2, ..., 2, 1] of turbo_simulator.py:778-781 and
 // turbo_main.py:2040-2044.  Bound by the FP64 pipe, so a thread takes the modes
 // kz and -kz together (one K2, one reciprocal root, one compensated addition
-// for both) and no division or square root: 36 FP64 instructions for two modes
-// where one took about 75.  N=2048: 421 us before, 98 now.
+// for both; what their own addition rounds off goes to the compensations) and
+// no division or square root: 46 FP64 instructions for two modes where one took
+// about 75.  N=2048: 421 us before, 98 now.
 template <typename T, int NT>
 __global__ void __launch_bounds__(NT) k_spectral(StepArgs a0) {
   using C = cplx<T>;
@@ -1866,28 +1876,33 @@ __global__ void __launch_bounds__(NT) k_spectral(StepArgs a0) {
     const C* __restrict__ col = om + (size_t)kx * N;
     const C o = col[kz];
     const double ox = widen(o.x), oy = widen(o.y);
-    double p = fma(ox, ox, oy * oy);
+    double p = fma(ox, ox, oy * oy), lo = 0.0;  // the pair's sum is p + lo
     bad |= !finite_bits(p);
     if (kz > 0 && kz < Nh) {
       const C q = col[N - kz];
       const double qx = widen(q.x), qy = widen(q.y);
       const double p2 = fma(qx, qx, qy * qy);
       bad |= !finite_bits(p2);
-      p += p2;
+      csum_add_pos(p, lo, p2);
     }
     const int k2 = kx * kx + kz * kz;
     const double K2 = double(k2);
-    const double pw = (kx == 0 || kx == Nh - 1) ? p : p + p;
+    const bool once = kx == 0 || kx == Nh - 1;
+    const double pw = once ? p : p + p, lw = once ? lo : lo + lo;
     if (k2 > 0) {
-      const double r = int_rsqrt(K2, k2);
-      const double e = pw * r * r;
+      const double r = int_rsqrt(K2, k2), ik = r * r;
+      const double e = over_k2(pw, K2, ik), el = lw * ik;
       csum_add_pos(s[0], c[0], e);
       csum_add_pos(s[1], c[1], e * r);
+      c[0] += el;
+      c[1] = fma(el, r, c[1]);
     } else {
       csum_add_pos(s[4], c[4], p);  // the (0,0) mode, removed from Z
     }
     csum_add_pos(s[2], c[2], pw);
     csum_add_pos(s[3], c[3], K2 * pw);
+    c[2] += lw;
+    c[3] = fma(K2, lw, c[3]);
   }
   __shared__ double red[2 * 5 * NT];
   block_csum<NT, 5>(s, c, red, tid);
@@ -1967,12 +1982,12 @@ __global__ void __launch_bounds__(NT) k_spectrum(const cplx<T>* __restrict__ om,
     if (kz > 0 && kz < Nh) {
       const cplx<T> q = col[N - kz];
       const double qx = widen(q.x), qy = widen(q.y);
-      p = fma(qx, qx, fma(qy, qy, p));
+      p += fma(qx, qx, qy * qy);
       n += wgt;
     }
     const int k2 = kx * kx + kz * kz;
-    const double r = int_rsqrt((double)k2, k2);
-    p = p * (r * r) * scale2;
+    const double K2 = (double)k2, r = int_rsqrt(K2, k2);
+    p = over_k2(p, K2, r * r) * scale2;
     e += wgt == 2 ? p + p : p;
   };
   int held = 0;
