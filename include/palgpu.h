@@ -169,7 +169,10 @@ int pal_fp64_peak(double* tflops, double* ms);
  * pal_create times them on the new handle and keeps the fastest, once per
  * (precision, N) per process; PAL_AUTOTUNE=0 in the environment keeps the
  * first candidates instead, and PAL_TMA_MULTICAST=0 leaves out the candidates
- * that load by TMA cluster multicast (N=8192 "... mc ...").  With
+ * that load by TMA cluster multicast (N=8192 "... mc ...").  A process of a job
+ * on several GPUs (more than one visible device, or WORLD_SIZE and the like
+ * above 1) never takes those, and pal_set_variant refuses them there with
+ * PAL_ERR_STATE.  With
  * PAL_TUNE_FILE=<path>, a size listed in that file
  * ("fp32 <N> <row name>|<column name>" per line) takes the named candidates
  * without timing and a timed size is appended, so that later processes run

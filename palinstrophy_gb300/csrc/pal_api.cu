@@ -280,6 +280,8 @@ int check(pal_handle* h) {
 int select_variant(pal_handle* h, int row, int col) {
   if (row < 0 || row >= h->ks->n_rows || col < 0 || col >= h->ks->n_cols)
     return fail(h, PAL_ERR_INVALID, "variant index out of range");
+  if (h->ks->rows[row].multicast && !pal::single_gpu_run())
+    return fail(h, PAL_ERR_STATE, "a row candidate with TMA multicast is for runs on one GPU alone");
   h->row_idx = row;
   h->col_idx = col;
   for (auto& kv : h->step_graphs) cudaGraphExecDestroy(kv.second);  // they hold the old kernels
@@ -311,8 +313,8 @@ std::map<std::pair<int, int>, std::pair<int, int>> g_tuned;
 // A size listed there takes the named candidates without timing; a size that
 // is timed is appended, so that later processes run the same kernels and give
 // bit-identical results.  Unknown names, other sizes and malformed lines are
-// skipped; a row candidate that loads by TMA multicast is skipped under
-// PAL_TMA_MULTICAST=0.
+// skipped, and so is a row candidate that loads by TMA multicast where that is
+// not allowed.
 const char* tune_file() {
   const char* f = std::getenv("PAL_TUNE_FILE");
   return (f && f[0]) ? f : nullptr;
@@ -369,7 +371,9 @@ int autotune(pal_handle* h) {
   std::lock_guard<std::mutex> lock(g_tune_mutex);
   {
     auto it = g_tuned.find(key);
-    if (it != g_tuned.end()) return select_variant(h, it->second.first, it->second.second);
+    // (a choice made before the process joined a job on several GPUs may have to go)
+    if (it != g_tuned.end() && (!h->ks->rows[it->second.first].multicast || pal::tma_multicast_allowed()))
+      return select_variant(h, it->second.first, it->second.second);
   }
   int best_row = 0, best_col = 0;
   if (tune_file_lookup(h, &best_row, &best_col)) {

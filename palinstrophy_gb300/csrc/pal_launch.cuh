@@ -26,7 +26,7 @@ struct RowKernels {
   void (*phys)(const StepArgs&, cudaStream_t);
   void (*twiddles)(void* tw, cudaStream_t);
   int (*blocks_per_sm)();  // resident k_row blocks per SM (occupancy calculator)
-  bool multicast = false;  // loads by TMA cluster multicast (left out of tuning by PAL_TMA_MULTICAST=0)
+  bool multicast = false;  // loads by TMA cluster multicast (tma_multicast_allowed)
 };
 
 struct ColKernels {
@@ -84,11 +84,23 @@ struct KernelSet {
   const AdjKernels* adj;  // nullptr where no adjoint is compiled
 };
 
-// Whether the autotuners may pick row candidates that load by TMA cluster
-// multicast: yes unless PAL_TMA_MULTICAST=0.
+// Whether this process is a run on one GPU alone: it sees one device, and no
+// launcher says that it is one of several processes (a job on several GPUs
+// usually gives each process one of them).
+inline bool single_gpu_run() {
+  for (const char* name : {"WORLD_SIZE", "LOCAL_WORLD_SIZE", "OMPI_COMM_WORLD_SIZE", "PMI_SIZE", "SLURM_NTASKS"}) {
+    const char* v = std::getenv(name);
+    if (v && std::atoi(v) > 1) return false;
+  }
+  int devices = 0;
+  return cudaGetDeviceCount(&devices) == cudaSuccess && devices == 1;
+}
+// Row candidates that load by TMA cluster multicast are for such runs only: a
+// job on several GPUs neither tunes to one nor may set one (pal_set_variant).
+// PAL_TMA_MULTICAST=0 keeps the autotuners off them on one GPU too.
 inline bool tma_multicast_allowed() {
   const char* e = std::getenv("PAL_TMA_MULTICAST");
-  return !(e && e[0] == '0');
+  return !(e && e[0] == '0') && single_gpu_run();
 }
 
 constexpr int kSpectralThreads = 256;

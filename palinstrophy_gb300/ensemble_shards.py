@@ -10,6 +10,7 @@ is no collective on the device.
 """
 from __future__ import annotations
 
+import os
 from typing import Sequence
 
 
@@ -62,6 +63,10 @@ def run_ensemble_shard(Ns: Sequence[int], seeds: Sequence[int], rank: int, world
     lo, hi = member_range(len(Ns), rank, world)
     if hi == lo:
         return []
+    if world > 1:
+        # one process of a job on several GPUs, whoever launched it: the library
+        # keeps its TMA multicast candidates to runs on one GPU alone
+        os.environ["PAL_TMA_MULTICAST"] = "0"
     ens = Ensemble(Ns[lo:hi], precision=precision, Re=Re, cfl=cfl)
     try:
         for m in range(hi - lo):
