@@ -59,10 +59,12 @@ __device__ __forceinline__ void fx_pass_tw(fxc (&x)[R], const int4* __restrict__
 #pragma unroll
   for (int k = 1; k < R; ++k) x[k] = fx_cmul4<(SIGN > 0)>(x[k], __ldg(t + (k - 1) * S));
 }
-// Bits of a pass's inputs: a DIT pass with twiddles divides them by 4 first.
+// Bits of a pass's inputs: a DIT pass with twiddles divides them by 4 first, but
+// multiplies them before it does, which has room for 62 bits (fx_cmul).
 template <class PL, int P, bool DIT>
 constexpr int fx_in_bits() {
-  return fx_bits(PL::R[P]) + (DIT && PL::stride(P) > 1 ? 2 : 0);
+  const int b = fx_bits(PL::R[P]);
+  return !(DIT && PL::stride(P) > 1) ? b : b + 2 < 62 ? b + 2 : 62;
 }
 template <class PL, int P>
 constexpr int fx_gain() {  // the pass's factor 2^-gain
