@@ -139,7 +139,10 @@ int pal_vis_field(pal_handle* h, int var, void* host_field, unsigned char* host_
  * the handle's fixed dt (no NEXTDT), with respect to the current om2 (the
  * velocity is taken as its inversion).  Hand-written discrete adjoint of the
  * stage (transposed padded transforms, adjoint products and inversion, reversed
- * IMEX stages), states checkpointed every ckpt_every steps and recomputed.
+ * IMEX stages), states checkpointed every ckpt_every steps and recomputed.  Device
+ * memory of a call, in planes of N/2 x 3N/2 complex values: 2 per checkpoint and 6
+ * per step between two of them; where that is more than 1 GiB the interval is
+ * sqrt(nsteps / 3) steps instead, which needs the least.
  * grad_host receives dL/d(om2) in the reference layout (real inner product
  * Re sum conj(g) d om2); the handle ends at the final forward state.  The
  * reference has no differentiation; N = 32..512.  Waits. */

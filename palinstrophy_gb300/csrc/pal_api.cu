@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "palgpu.h"
+#include "pal_segments.h"
 #include "pal_launch.cuh"
 
 using pal::ColKernels;
@@ -913,12 +914,8 @@ int pal_adjoint_palinstrophy(pal_handle* h, int nsteps, int ckpt_every, double* 
   if (h->state != ST_U) return fail(h, PAL_ERR_STATE, "adjoint needs the physical velocity");
   if (adj->configure() != cudaSuccess) return fail(h, PAL_ERR_CUDA, "adjoint configure");
   const size_t plane_om = (size_t)h->Nh * h->N * h->esz, plane_w = (size_t)h->Nh * h->M * h->esz;
-  // Segments of `seg` steps: their stages' velocity planes (two of plane_w each)
-  // are kept while the segment runs backward.  ckpt_every steps, or a third of
-  // that where the planes would take more than 1 GiB (they are three times the
-  // stage's om; a shorter segment costs checkpoints, not recomputation).
-  const size_t per_step = 3 * 2 * plane_w;
-  const int seg = std::min(nsteps, (size_t)ckpt_every * per_step <= ((size_t)1 << 30) ? ckpt_every : (ckpt_every + 2) / 3);
+  const size_t per_step = 3 * 2 * plane_w;  // the velocity planes of a step's stages
+  const int seg = pal::adjoint_segment(nsteps, ckpt_every, plane_w);
   const int n_ck = (nsteps + seg - 1) / seg;
   // one allocation: checkpoints (om, fnm1, butterfly-major) of all segments but the last |
   // velocity planes of a segment's stages and of its end | om, fnm1 of the segment, lam_om, lam_f |
