@@ -104,6 +104,10 @@ __host__ __device__ constexpr int fx_lo(long long v) { return (int)(v - ((long l
 __host__ __device__ constexpr int fx_bits(int R) {
   return R <= 2 ? 61 : R <= 4 ? 60 : R <= 8 ? 59 : R <= 16 ? 58 : 57;
 }
+// The same for the first pass over a line with the 3/2 pad: a butterfly of a
+// radix R divisible by 3 has R / 3 zeros among its inputs (the middle third, in
+// natural order for the first radix and in digit-reversed for the last).
+__host__ __device__ constexpr int fx_pad_bits(int R) { return fx_bits(R % 3 == 0 ? 2 * R / 3 : R); }
 
 // Multiply by W_R^(SIGN*E), all compile time (the integer counterpart of twc).
 template <int R, int E, int SIGN>

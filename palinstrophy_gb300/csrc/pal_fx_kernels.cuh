@@ -121,10 +121,10 @@ __device__ __forceinline__ double fx_speed_value(unsigned long long top, FxScale
 }
 
 // One pass over a [slot][v] tile.  RAW: the tile is FP64 with the largest
-// exponent `s`, else integers to be shifted by `s`.  PAD: positions N/2 ..
-// M - N/2 of the lines are zero (the 3/2 pad): whole segments are not read.
-// Returns the largest word of the outputs.
-template <class PL, int V, int NT, int P, int SIGN, bool DIT, bool RAW, bool PAD = false>
+// exponent `s`, taken to K bits, else integers to be shifted by `s`.  PAD:
+// positions N/2 .. M - N/2 of the lines are zero (the 3/2 pad): whole segments
+// are not read.  Returns the largest word of the outputs.
+template <class PL, int V, int NT, int P, int SIGN, bool DIT, bool RAW, bool PAD = false, int K = fx_bits(PL::R[P])>
 __device__ __forceinline__ unsigned fx_pass(fxc* sm, const int4* __restrict__ tw, int tid, int s, bool bad) {
   constexpr int R = PL::R[P];
   constexpr int L = PL::span(P);
@@ -146,7 +146,7 @@ __device__ __forceinline__ unsigned fx_pass(fxc* sm, const int4* __restrict__ tw
         x[k] = fxc{0, 0};
       } else if constexpr (RAW) {
         const double2 d = fx_unraw(p[k * SP * V]);
-        x[k] = bad ? fxc{0, 0} : fxc{fx_from_double<fx_bits(R)>(d.x, s), fx_from_double<fx_bits(R)>(d.y, s)};
+        x[k] = bad ? fxc{0, 0} : fxc{fx_from_double<K>(d.x, s), fx_from_double<K>(d.y, s)};
       } else {
         x[k] = p[k * SP * V];
       }
@@ -198,7 +198,12 @@ __device__ __forceinline__ void fx_rows_inverse(const void* p0, const void* p1, 
                                                 int z0, int tid, FxWords* ws, FxScale& sc) {
   constexpr int M = PL::M, Nh = M / 3;
   constexpr int CNT = (Nh * V + NT - 1) / NT;
-  constexpr int K = fx_bits(PL::R[0]) - 1;  // Z is a sum of two
+  // Z is a sum of two, of values taken to half units and rounded to nearest: a
+  // row with a few large values and many small ones loses most here, at the
+  // tile's unit.  With values truncated at fx_bits - 1 a velocity of spectrum
+  // k^-2 was 3.0, 3.1 and 3.8 to 6.1e-16 off at N = 1024, 2048 and 4096, where
+  // FP64 transforms are 2.4, 2.8 and 3.3e-16 off and this is 1.4, 2.3 and 2.7.
+  constexpr int K = fx_pad_bits(PL::R[0]);
   const double2* __restrict__ w0 = static_cast<const double2*>(p0);
   const double2* __restrict__ w1 = static_cast<const double2*>(p1);
   fx_words_clear<NT>(ws, tid);
@@ -220,7 +225,7 @@ __device__ __forceinline__ void fx_rows_inverse(const void* p0, const void* p1, 
   for (int w = tid; w < V * (M - 2 * Nh + 1); w += NT) sm[PL::phys(Nh + w / V) * V + w % V] = fxc{0, 0};
   __syncthreads();
   const int emax = fx_emax(ws->top[0]);
-  sc = FxScale{fx_exponent(emax, K), emax == 0x7ff};
+  sc = FxScale{fx_exponent(emax, K) + 1, emax == 0x7ff};
 #pragma unroll
   for (int c = 0; c < CNT; ++c) {
     const int w = tid + c * NT;
@@ -233,8 +238,9 @@ __device__ __forceinline__ void fx_rows_inverse(const void* p0, const void* p1, 
         qx = fx_from_double<K>(q[c].x, emax);
         qy = fx_from_double<K>(q[c].y, emax);
       }
-      sm[PL::phys(k) * V + v] = k == 0 ? fxc{ux, qx} : fxc{ux - qy, uy + qx};
-      if (k > 0) sm[PL::phys(M - k) * V + v] = fxc{ux + qy, qx - uy};
+      if (k == 0) uy = qy = 0;
+      sm[PL::phys(k) * V + v] = fxc{(ux - qy + 1) >> 1, (uy + qx + 1) >> 1};
+      if (k > 0) sm[PL::phys(M - k) * V + v] = fxc{(ux + qy + 1) >> 1, (qx - uy + 1) >> 1};
     }
   }
   __syncthreads();
@@ -424,13 +430,16 @@ __device__ __forceinline__ FxScale fx_column_forward(fxc* sm, const int4* __rest
 
 // The inverse z-transform of a raw column tile (A tile of two lines in
 // digit-reversed order, its largest high word in top[SLOT]) into the U planes.
+// Its first pass is over the lines' pad: with RP divisible by 3 the middle third
+// of every butterfly's inputs is zero (fx_pad_bits).
 template <class PL, int NT, int SLOT>
 __device__ __forceinline__ void fx_column_inverse(fxc* sm, const int4* __restrict__ tw, double2* __restrict__ w0,
                                                   double2* __restrict__ w1, int kx, int tid, FxWords* ws) {
   constexpr int M = PL::M, V = 2, NP = PL::NP;
   const int emax = fx_emax(ws->top[SLOT]);
-  FxScale sc{fx_exponent(emax, fx_bits(PL::RP)), emax == 0x7ff};
-  fx_note(fx_pass<PL, V, NT, NP - 1, +1, true, true>(sm, tw, tid, emax, sc.bad), &ws->bits[2 * NP - 1], tid);
+  constexpr int K = fx_pad_bits(PL::RP);
+  FxScale sc{fx_exponent(emax, K), emax == 0x7ff};
+  fx_note(fx_pass<PL, V, NT, NP - 1, +1, true, true, false, K>(sm, tw, tid, emax, sc.bad), &ws->bits[2 * NP - 1], tid);
   __syncthreads();
   fx_dit<PL, V, NT, +1, NP - 2, 1, NP>(sm, tw, tid, ws, sc);
   // the last pass straight into the planes

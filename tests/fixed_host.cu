@@ -1,5 +1,6 @@
-// Prints "R fx_bits in_dit" for every radix that a plan can be built of: the
-// bits of the inputs of a pass without and, in a DIT pass, before its twiddles.
+// Prints "R fx_bits in_dit pad" for every radix that a plan can be built of: the
+// bits of the inputs of a pass without and, in a DIT pass, before its twiddles,
+// and those of the first pass over a padded line.
 #include <cstdio>
 
 #include "pal_fx_kernels.cuh"
@@ -7,7 +8,7 @@
 template <int R>
 void line() {
   using PL = pal::FxPlan<pal::Plan<12 * R, R, 12>>;
-  std::printf("%d %d %d\n", R, pal::fx_bits(R), pal::fx_in_bits<PL, 0, true>());
+  std::printf("%d %d %d %d\n", R, pal::fx_bits(R), pal::fx_in_bits<PL, 0, true>(), pal::fx_pad_bits(R));
 }
 
 int main() {

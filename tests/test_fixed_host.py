@@ -18,7 +18,10 @@ def test_no_pass_leaves_64_bits(tmp_path):
     rows = [tuple(map(int, ln.split())) for ln in
             subprocess.run([exe], capture_output=True, text=True, check=True).stdout.splitlines()]
     assert len(rows) == 9
-    for R, b, b_dit in rows:
+    for R, b, b_dit, b_pad in rows:
+        # positions N/2 .. M - N/2 of a padded line are zero: segment j of R holds (3 j .. 3 j + 3) N / 2R
+        inputs = sum(not (3 * j >= R and 3 * j + 3 <= 2 * R) for j in range(R))
+        assert math.log2(inputs) + b_pad + 0.5 <= 62.8, R
         assert math.log2(R) + b + 0.5 <= 62.8, R
         assert b_dit + 0.5 <= 62.8, R   # what the DIT twiddles multiply
         assert b_dit - 2 <= b, R        # they divide by 4
