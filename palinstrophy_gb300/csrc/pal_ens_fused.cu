@@ -144,19 +144,22 @@ struct FusedOf {
 // blocks per SM) for either pass: 286.  The passes are bound by issue and
 // latency, not by memory: stepping quarters of the members one after the other,
 // whose state then stays in L2, took 320, the gain lost to the launches' tails.
+// Columns of N=384 and 512 have full twiddle tables after the first pass, which
+// costs no time and halves what twiddles formed in registers add to the rounding
+// at high wave numbers (pal_inst_f32_e.cu).
 using P384 = Plan<384, 6, 8, 8>;
 using P576 = Plan<576, 6, 8, 12>;
 using P768 = Plan<768, 8, 8, 12>;
 using S256 = FusedSize<Rec<P384>, 4, 14, Rec<P384>, 2>;
-using S384 = FusedSize<Rec<P576>, 4, 14, Rec<P576>, 2>;
-using S512 = FusedSize<Rec<P768>, 4, 14, Rec<P768>, 2>;
+using S384 = FusedSize<Rec<P576>, 4, 14, RecT<P576>, 2>;
+using S512 = FusedSize<Rec<P768>, 4, 14, RecT<P768>, 2>;
 using F3 = FusedOf<192, 64, S256, S384, S512>;
 
 const FusedSet kSet3 = {3,
                         {256, 384, 512},
                         {"6.8.8r V4x192 tma-in tma-out", "6.8.12r V4x192 tma-in tma-out",
                          "8.8.12r V4x192 tma-in tma-out"},
-                        {"6.8.8r x128 hoist", "6.8.12r x192 hoist", "8.8.12r x192 hoist"},
+                        {"6.8.8r x128 hoist", "6.8.12t x192 hoist", "8.8.12t x192 hoist"},
                         {4, 4, 4},
                         192,
                         F3::smem_row,

@@ -49,10 +49,13 @@ const ColKernels c256[] = {ColOf<float, P384, 128>::make("16.24 x128"), ColOf<fl
                            ColOf<float, Rec<P384>, 128, 2>::make("16.24r x128 hoist"),
                            ColOf<float, Rec<P384b>, 128, 2>::make("24.16r x128 hoist"),
                            ColOf<float, Rec<P384d>, 128, 2>::make("6.8.8r x128 hoist")};
+// Adjoint on full tables: twiddles formed in registers (Rec) raised the error of
+// the gradient of a steep field, N=128 9.6e-6 -> 1.3e-5, N=256 1.6e-4 -> 2.5e-4;
+// 1.39 and 1.74 ms for 20 steps (1.33 and 1.75 with Rec).
 PAL_KERNEL_SET_ADJ(float, 0, 32, r32, c32, (AdjOf<float, P48, 4, 64, P48, 64>::get()))
 PAL_KERNEL_SET_ADJ(float, 0, 64, r64, c64, (AdjOf<float, P96, 4, 128, P96, 64>::get()))
-PAL_KERNEL_SET_ADJ(float, 0, 128, r128, c128, (AdjOf<float, Rec<P192>, 4, 128, Rec<P192>, 64>::get()))
-PAL_KERNEL_SET_ADJ(float, 0, 256, r256, c256, (AdjOf<float, Rec<P384>, 4, 128, Rec<P384c>, 96>::get()))
+PAL_KERNEL_SET_ADJ(float, 0, 128, r128, c128, (AdjOf<float, P192, 4, 128, P192, 64>::get()))
+PAL_KERNEL_SET_ADJ(float, 0, 256, r256, c256, (AdjOf<float, P384, 4, 128, P384c, 96>::get()))
 }  // namespace
 
 const KernelSet* pal_kernels_f32_a(int N) {

@@ -1,8 +1,9 @@
 // FP32 candidates, N = 2048 and 3072 (M = 3072, 4608).
 //
-// N=3072 columns: 24.16.12 on 288 threads 109.5 us, against 112.2 with
-// 16.12.24 on 256; at N=2048 16.16.12 is no faster than 8.16.24 (43.4 us both),
-// and 24.16.12 is slower for the rows of N=3072.
+// Tried: N=2048 columns 16.16.12, no faster than 8.16.24 (43.4 us both); N=3072
+// columns 24.16.12 on 288 threads, 109.9 us with formed twiddles but 1.42 times
+// the K2-weighted error of full tables (16.12.24r: 112.9 us, 1.24), 112.2 us with
+// full tables after the first pass; 24.16.12 is slower for the rows of N=3072.
 #include "pal_launch.cuh"
 
 using namespace pal;
@@ -10,7 +11,6 @@ using namespace pal;
 namespace {
 using P3072 = Plan<3072, 16, 8, 24>;
 using P3072b = Plan<3072, 8, 16, 24>;
-using P4608c = Plan<4608, 24, 16, 12>;
 using P4608 = Plan<4608, 16, 12, 24>;
 
 const RowKernels r2048[] = {RowOf<float, P3072, 4, 512>::make("16.8.24 V4x512"),
@@ -43,8 +43,7 @@ const RowKernels r3072[] = {RowOf<float, P4608, 4, 512>::make("16.12.24 V4x512")
 const ColKernels c3072[] = {ColOf<float, P4608, 256>::make("16.12.24 x256"), ColOf<float, P4608, 512>::make("16.12.24 x512"),
                             ColOf<float, Rec<P4608>, 256>::make("16.12.24r x256"),
                             ColOf<float, Rec<P4608>, 256, 2>::make("16.12.24r x256 hoist"),
-                            ColOf<float, Rec<P4608>, 256, 4>::make("16.12.24r x256 tma"),
-                            ColOf<float, Rec<P4608c>, 288, 4>::make("24.16.12r x288 tma")};
+                            ColOf<float, Rec<P4608>, 256, 4>::make("16.12.24r x256 tma")};
 
 PAL_KERNEL_SET(float, 0, 2048, r2048, c2048)
 PAL_KERNEL_SET(float, 0, 3072, r3072, c3072)

@@ -8,6 +8,13 @@
 // last candidate of each list: columns N=384 12.2 -> 10.8, 512 12.6 -> 11.9,
 // 768 16.2 -> 14.1; rows 512 10.54 -> 10.45, 384 and 768 the same with 6.8.12
 // and 8.12.12 (8.45, 12.6: not listed).
+//
+// Twiddles formed in registers (Rec) add rounding that grows with the number of
+// passes and shows at high wave numbers.  K2-weighted error of five RK3 steps
+// over that of full tables: columns 24.24r 1.26, 6.8.12r 1.40, 6.8.12t 1.09;
+// 32.24r 1.25, 8.8.12r 1.49, 8.8.12t 1.15.  So these columns have full tables
+// after the first pass (RecT), at the same time: 10.59 and 10.76 us a launch
+// (10.56 and 10.78 with Rec).
 #include "pal_launch.cuh"
 
 using namespace pal;
@@ -35,7 +42,7 @@ const RowKernels r384[] = {RowOf<float, P576, 4, 256>::make("24.24 V4x256"),
                            RowOf<float, Rec<P576c>, 4, 192, 14>::make("6.8.12r V4x192 tma-in tma-out")};
 const ColKernels c384[] = {ColOf<float, P576, 128>::make("24.24 x128"), ColOf<float, P576b, 128>::make("6.6.16 x128"),
                            ColOf<float, Rec<P576>, 128, 2>::make("24.24r x128 hoist"),
-                           ColOf<float, Rec<P576c>, 192, 2>::make("6.8.12r x192 hoist")};
+                           ColOf<float, RecT<P576c>, 192, 2>::make("6.8.12t x192 hoist")};
 const RowKernels r512[] = {RowOf<float, P768, 4, 256>::make("32.24 V4x256"),
                            RowOf<float, P768, 2, 128>::make("32.24 V2x128"),
                            RowOf<float, P768b, 4, 256>::make("16.2.24 V4x256"),
@@ -52,7 +59,7 @@ const ColKernels c512[] = {ColOf<float, P768, 128>::make("32.24 x128"), ColOf<fl
                            ColOf<float, Rec<P768>, 128, 2>::make("32.24r x128 hoist"),
                            ColOf<float, Rec<P768b>, 128, 2>::make("16.2.24r x128 hoist"),
                            ColOf<float, Rec<P768b>, 128, 4>::make("16.2.24r x128 tma"),
-                           ColOf<float, Rec<P768c>, 192, 2>::make("8.8.12r x192 hoist")};
+                           ColOf<float, RecT<P768c>, 192, 2>::make("8.8.12t x192 hoist")};
 const RowKernels r768[] = {RowOf<float, P1152, 4, 256>::make("8.6.24 V4x256"),
                            RowOf<float, P1152, 2, 256>::make("8.6.24 V2x256"),
                            RowOf<float, P1152b, 4, 256>::make("12.4.24 V4x256"),
@@ -67,7 +74,9 @@ const ColKernels c768[] = {ColOf<float, P1152, 256>::make("8.6.24 x256"), ColOf<
                            ColOf<float, Rec<P1152c>, 192, 4>::make("8.12.12r x192 tma")};
 
 PAL_KERNEL_SET(float, 0, 384, r384, c384)
-PAL_KERNEL_SET_ADJ(float, 0, 512, r512, c512, (AdjOf<float, Rec<P768c>, 4, 384, Rec<P768c>, 192>::get()))
+// Adjoint on full tables for the same reason, gradient of a steep field: error
+// 2.7e-3, 3.7e-3 with Rec; 2.63 ms for 20 steps, 2.71.
+PAL_KERNEL_SET_ADJ(float, 0, 512, r512, c512, (AdjOf<float, P768c, 4, 384, RecT<P768c>, 192>::get()))
 PAL_KERNEL_SET(float, 0, 768, r768, c768)
 }  // namespace
 
