@@ -120,16 +120,22 @@ bool encode_row_maps(TmaMaps* out, void* w0, void* w1, int N, int V, int members
 // box, so one box row is a padded group of ColPlanar.
 bool encode_col_maps(TmaMaps* out, void* w0, void* w1, int N, int RP, int members);
 
-// Launch of a kernel that begins with pdl_wait() (its EARLY the same): with
+// Launch of a kernel that begins with pdl_wait() where EARLY is set: with
 // EARLY the stream may bring its blocks onto the GPU while the previous kernel's
 // last ones run, which saves the launch between two kernels (about 1.5 us).  The
 // blocks that wait hold their SM's registers and shared memory, though, and
 // where several streams share the GPU with small kernels that costs more: three
 // N=256 FP64 fields side by side took 372 us a call with it and 293 without.  So
-// early launches are for FP32 passes of several waves (kEarlyM: N=4096 RK3 3.50
-// ms for four steps, 3.55 without; one N=1536 field alone 1.77 ms for ten, 1.92
-// without) and for the adjoint's short dependent launches (N=512 gradient 3.82
-// ms, 4.36 without).
+// early launches are for
+// - FP32 passes of several waves (kEarlyM: N=4096 RK3 3.50 ms for four steps,
+//   3.55 without; one N=1536 field alone 1.77 ms for ten, 1.92 without);
+// - the adjoint's short dependent launches, but for FP64 from N=256 on (AdjOf).
+//   ms for 20 steps, one gradient alone / three side by side in threads, with
+//   early launches and without: FP32 N=32 1.02 / 1.09 and 1.67 / 1.98, N=128
+//   1.39 / 1.51 and 2.19 / 2.37, N=256 1.75 / 2.18 and 2.27 / 2.91, N=512 2.61 /
+//   3.60 and 3.21 / 3.89; FP64 N=32 2.77 / 2.85 and 3.24 / 3.73, N=128 3.48 /
+//   4.44 and 3.88 / 4.65, N=256 4.38 / 6.62 and 4.38 / 6.02, N=512 9.78 / 14.5
+//   and 8.32 / 14.1.
 template <bool EARLY, class... P, class... A>
 inline void launch_pdl(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, const A&... args) {
   cudaLaunchConfig_t cfg = {};
@@ -414,6 +420,7 @@ struct ColFxOf {
 template <typename T, class PLR, int V, int NTR, class PLC, int NTC>
 struct AdjOf {
   static constexpr bool FX = std::is_same_v<T, double>;
+  static constexpr bool EARLY = !FX || PLC::M < 384;
   static constexpr size_t smem_fwd = size_t(PLR::PADM) * V * sizeof(cplx<T>);
   static constexpr size_t smem_row = 2 * smem_fwd;  // the lam and the velocity tile
   static constexpr size_t smem_col = size_t(PLC::PADM) * 2 * sizeof(cplx<T>);
@@ -441,42 +448,42 @@ struct AdjOf {
   }
   static void vel(const StepArgs& a, cudaStream_t s) {
     if constexpr (FX)
-      launch_pdl<true>(k_adj_vel_fx<FxPlan<PLC>, NTC>, N / 2, NTC, smem_col, s, a);
+      launch_pdl<EARLY>(k_adj_vel_fx<FxPlan<PLC>, NTC>, N / 2, NTC, smem_col, s, a);
     else
-      launch_pdl<true>(k_adj_vel<T, PLC, NTC>, N / 2, NTC, smem_col, s, a);
+      launch_pdl<EARLY>(k_adj_vel<T, PLC, NTC>, N / 2, NTC, smem_col, s, a);
   }
   static void fwd_row(const StepArgs& a, cudaStream_t s) {
     if constexpr (FX)
-      launch_pdl<true>(k_adj_fwd_row_fx<FxPlan<PLR>, V, NTR>, PLR::M / V, NTR, smem_fwd, s, a);
+      launch_pdl<EARLY>(k_adj_fwd_row_fx<FxPlan<PLR>, V, NTR>, PLR::M / V, NTR, smem_fwd, s, a);
     else
-      launch_pdl<true>(k_adj_fwd_row<T, PLR, V, NTR>, PLR::M / V, NTR, smem_fwd, s, a);
+      launch_pdl<EARLY>(k_adj_fwd_row<T, PLR, V, NTR>, PLR::M / V, NTR, smem_fwd, s, a);
   }
   static void fwd_col(const StepArgs& a, cudaStream_t s) {
     if constexpr (FX)
-      launch_pdl<true>(k_adj_fwd_col_fx<FxPlan<PLC>, NTC>, N / 2, NTC, smem_col, s, a);
+      launch_pdl<EARLY>(k_adj_fwd_col_fx<FxPlan<PLC>, NTC>, N / 2, NTC, smem_col, s, a);
     else
-      launch_pdl<true>(k_adj_fwd_col<T, PLC, NTC>, N / 2, NTC, smem_col, s, a);
+      launch_pdl<EARLY>(k_adj_fwd_col<T, PLC, NTC>, N / 2, NTC, smem_col, s, a);
   }
   static void col(const StepArgs& a, cudaStream_t s) {
     if constexpr (FX)
-      launch_pdl<true>(k_adj_col_fx<FxPlan<PLC>, NTC>, N / 2, NTC, smem_col, s, a);
+      launch_pdl<EARLY>(k_adj_col_fx<FxPlan<PLC>, NTC>, N / 2, NTC, smem_col, s, a);
     else
-      launch_pdl<true>(k_adj_col<T, PLC, NTC>, N / 2, NTC, smem_col, s, a);
+      launch_pdl<EARLY>(k_adj_col<T, PLC, NTC>, N / 2, NTC, smem_col, s, a);
   }
   static void row(const StepArgs& a, cudaStream_t s) {
     if constexpr (FX)
-      launch_pdl<true>(k_adj_row_fx<FxPlan<PLR>, V, NTR>, PLR::M / V, NTR, smem_row, s, a);
+      launch_pdl<EARLY>(k_adj_row_fx<FxPlan<PLR>, V, NTR>, PLR::M / V, NTR, smem_row, s, a);
     else
-      launch_pdl<true>(k_adj_row<T, PLR, V, NTR>, PLR::M / V, NTR, smem_row, s, a);
+      launch_pdl<EARLY>(k_adj_row<T, PLR, V, NTR>, PLR::M / V, NTR, smem_row, s, a);
   }
   static void seed(const void* om, void* lom, void* lf, double* loss_part, cudaStream_t s) {
     k_adj_seed<T, PLC, 128><<<N / 2, 128, 0, s>>>(static_cast<const cplx<T>*>(om), static_cast<cplx<T>*>(lom),
                                                   static_cast<cplx<T>*>(lf), loss_part);
   }
   static dim3 grid_perm(const StepArgs& a) { return dim3(N / 2, 1, (a.flags & F_NO_FM_IN) ? 1 : 2); }
-  static void to_perm(const StepArgs& a, cudaStream_t s) { launch_pdl<true>(k_om_perm<T, PLC, true, true>, grid_perm(a), 256, smem_perm, s, a); }
+  static void to_perm(const StepArgs& a, cudaStream_t s) { launch_pdl<EARLY>(k_om_perm<T, PLC, true, true>, grid_perm(a), 256, smem_perm, s, a); }
   static void from_perm(const StepArgs& a, cudaStream_t s) {
-    launch_pdl<true>(k_om_perm<T, PLC, false, true>, grid_perm(a), 256, smem_perm, s, a);
+    launch_pdl<EARLY>(k_om_perm<T, PLC, false, true>, grid_perm(a), 256, smem_perm, s, a);
   }
   static const AdjKernels* get() {
     if constexpr (FX) {
