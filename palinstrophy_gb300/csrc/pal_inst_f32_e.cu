@@ -6,7 +6,7 @@
 // loads in flight, shorter serial butterflies) beats fewer, larger passes.
 // us per launch with the launch itself (about 4.5), GB300, before -> with the
 // last candidate of each list: columns N=384 12.2 -> 10.8, 512 12.6 -> 11.9,
-// 768 16.2 -> 14.1; rows 512 10.54 -> 10.45, 384 and 768 the same with 6.8.12
+// 768 16.2 -> 14.1; rows 512 10.59 -> 10.50, 384 and 768 the same with 6.8.12
 // and 8.12.12 (8.45, 12.6: not listed).
 //
 // Twiddles formed in registers (Rec) add rounding that grows with the number of
@@ -52,7 +52,6 @@ const RowKernels r512[] = {RowOf<float, P768, 4, 256>::make("32.24 V4x256"),
                            RowOf<float, Rec<P768b>, 4, 256, 15>::make("16.2.24r V4x256 tma-in tma-out l2pf"),
                            RowOf<float, Rec<P768>, 4, 128, 15>::make("32.24r V4x128 tma-in tma-out l2pf"),
                            RowOf<float, Rec<P768b>, 4, 128, 14>::make("16.2.24r V4x128 tma-in tma-out"),
-                           RowOf<float, Rec<P768c>, 2, 192, 2>::make("8.8.12r V2x192 paired"),
                            RowOf<float, Rec<P768c>, 4, 192, 14>::make("8.8.12r V4x192 tma-in tma-out")};
 const ColKernels c512[] = {ColOf<float, P768, 128>::make("32.24 x128"), ColOf<float, P768b, 128>::make("16.2.24 x128"),
                            ColOf<float, P768, 256>::make("32.24 x256"),

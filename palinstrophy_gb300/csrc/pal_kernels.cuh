@@ -427,14 +427,13 @@ __device__ __forceinline__ NextDt nextdt_from_mark(const StepArgs& a) {
 // Z[k] = u^[k] + i v^[k] (k < N/2; real parts only at k = 0),
 // Z[M-k] = conj(u^[k]) + i conj(v^[k]), zero elsewhere (the 3/2 pad).
 template <typename T, class PL, int V, int NT>
-__device__ __forceinline__ void row_first_pass(const StepArgs& a, cplx<T>* sm, int z0, int tid,
-                                               const void* p0 = nullptr, const void* p1 = nullptr) {
+__device__ __forceinline__ void row_first_pass(const StepArgs& a, cplx<T>* sm, int z0, int tid) {
   using C = cplx<T>;
   constexpr int M = PL::M;
   constexpr int R = PL::R[0];
   constexpr int S = M / R;
-  const C* __restrict__ w0 = static_cast<const C*>(p0 ? p0 : a.w0);
-  const C* __restrict__ w1 = static_cast<const C*>(p1 ? p1 : a.w1);
+  const C* __restrict__ w0 = static_cast<const C*>(a.w0);
+  const C* __restrict__ w1 = static_cast<const C*>(a.w1);
   const C* __restrict__ tw = static_cast<const C*>(a.tw);
   constexpr int Nh = M / 3;
   for (int w = tid; w < V * S; w += NT) {
