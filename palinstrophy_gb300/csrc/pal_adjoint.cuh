@@ -29,7 +29,7 @@
 // Small grids are bound by the latency of the passes and launches: N=512 FP32,
 // 200 steps 40.2 ms before (natural-order columns, the stage inputs copied, the
 // velocity transformed again, seven launches a stage), 23.9 ms now; FP64 20
-// steps 37.1 and 9.0 ms.
+// steps 37.1 and 8.3 ms.
 #pragma once
 #include "pal_kernels.cuh"
 

@@ -737,7 +737,7 @@ int pal_step(pal_handle* h, int method, int nsteps, int update, int final_update
       pending = update > 0 && (it % update == 0 || it == 1 || (final_update && j == nsteps));
     }
     // The column pass runs on the butterfly-major om order, whose two
-    // conversions (~60 us each at N=4096) cost less than one step's three
+    // conversions (24 and 35 us at N=4096) cost less than one step's three
     // natural-order column passes (~370 us more).
     auto record = [&]() -> int {
       if (int rc = om_layout(h, true, method)) return rc;

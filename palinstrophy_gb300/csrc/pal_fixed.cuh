@@ -6,10 +6,14 @@
 // two to integers below 2^K, every pass of the transform runs in integers, and
 // between passes the tile is shifted back below 2^K (the largest magnitude
 // says by how much).  K leaves room for the growth of one pass, so no sum can
-// overflow, and the unit is 2^-57 .. 2^-60 of the line's largest value where
-// FP64 rounds at 2^-53 of each value: the error of a transform, relative to
-// its line, is below that of the FP64 transform it replaces (measured against
-// 80-bit arithmetic in tests/test_gpu_kernels.py).
+// overflow: fx_bits and fx_pad_bits by the pass's radix, and a tile one bit
+// short of it stays as it is, so the unit is 2^-56 (radices 9 to 16) to 2^-61
+// of the tile's largest value.  (A tile holds one to four lines, which share the
+// exponent.)  FP64 rounds at 2^-53 of each value instead: small values beside
+// large ones keep fewer digits here, but the error of a transform relative to
+// its tile is below that of the FP64 transform it replaced on random-phase
+// spectra from white to k^-2 (against long double; tests/test_gpu_kernels.py and
+// test_gpu_fixed_point.py).
 //
 // Constants and twiddles are 62-bit fractions split into 32-bit halves with a
 // signed low half.  A product keeps the three larger partial products (the

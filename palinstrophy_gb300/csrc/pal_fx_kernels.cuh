@@ -272,10 +272,10 @@ __device__ __forceinline__ void fx_rows_unpack(void* p0, void* p1, const fxc* sm
 }
 
 // k_row in fixed point: U-state rows -> products -> P-state rows, optional CFL
-// statistics.  Bound by the integer pipes (ncu: ALU 55 % of its rate, the
-// widening multiply-adds most of the rest) and, with one or two tiles per SM, by
-// the latency between its passes.  N=4096 1190 us (FP64 transforms: 6120, the
-// FP64 pipe 83 % busy), N=1024 70 us (352).
+// statistics.  No pipe is full (ncu, N=4096: issue 46 %, integer ALU 50 %, the
+// FMA pipe that runs the widening multiply-adds 24 %): with one or two tiles per
+// SM the latency of loads, passes and barriers in turn bounds it.  N=4096 1191 us
+// (FP64 transforms: 6120, the FP64 pipe 83 % busy), N=1024 72 us (352).
 template <class PL, int V, int NT>
 __device__ __forceinline__ void row_fx_body(const StepArgs& a, const void* u0, const void* u1, const Blk bk) {
   extern __shared__ __align__(128) unsigned char smraw[];
@@ -467,7 +467,7 @@ __device__ __forceinline__ void fx_column_inverse(fxc* sm, const int4* __restric
 // The update between the transforms is FP64, 28 to 32 FP64 instructions a mode:
 // reciprocals in four, the scale 1 / M^2 in the stage's weights, wave-number
 // products in integers (exact: N is at most 4096).  PERM and the stage flags as
-// k_col.  N=4096 1210 us (FP64 transforms: 4300), N=1024 78 us (317).
+// k_col.  N=4096 1225 us (FP64 transforms: 4300), N=1024 81 us (317).
 template <class PL, int NT, bool PERM>
 __device__ __forceinline__ void col_fx_body(const StepArgs& a, void* d0, void* d1, const Blk bk) {
   static_assert(PL::M <= 6144, "K2 within 24 bits (fx_small)");

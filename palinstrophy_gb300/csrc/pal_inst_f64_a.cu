@@ -1,5 +1,8 @@
 // FP64 candidates, N = 32 .. 512, with fixed-point transforms
-// (pal_fx_kernels.cuh, pal_fx_adjoint.cuh).
+// (pal_fx_kernels.cuh, pal_fx_adjoint.cuh).  us per launch with the launch
+// itself, first and second of a list, GB300: columns N=32 16.17 and 16.25, 256
+// 20.1 and 21.9; rows 512 22.6 and 22.7.  The second ones are near enough to
+// trade places on a shared GPU.
 #include "pal_launch.cuh"
 
 using namespace pal;

@@ -1,5 +1,6 @@
 // FP64 candidates, N = 2048 and 3072, with fixed-point transforms
-// (pal_fx_kernels.cuh).
+// (pal_fx_kernels.cuh).  us per launch, first and second of a list, GB300: rows
+// N=2048 296 and 295, 3072 757 and 755; columns 2048 271 and 288.
 #include "pal_launch.cuh"
 
 using namespace pal;

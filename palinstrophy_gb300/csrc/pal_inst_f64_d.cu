@@ -1,5 +1,6 @@
 // FP64 candidates, N = 4096, with fixed-point transforms
-// (pal_fx_kernels.cuh).
+// (pal_fx_kernels.cuh).  us per launch, first and second of a list, GB300: rows
+// 1243 and 1230, columns 1268 and 1302.
 #include "pal_launch.cuh"
 
 using namespace pal;

@@ -1857,7 +1857,8 @@ __device__ __forceinline__ double over_k2(double p, double K2, double ik) {
 // kz and -kz together (one K2, one reciprocal root, one compensated addition
 // for both; what their own addition rounds off goes to the compensations) and
 // no division or square root: 46 FP64 instructions for two modes where one took
-// about 75.  N=2048: 421 us before, 98 now.
+// about 75.  N=2048: 421 us before, 119 now (98 with the products and the pairs'
+// sums rounded).
 template <typename T, int NT>
 __global__ void __launch_bounds__(NT) k_spectral(StepArgs a0) {
   using C = cplx<T>;
@@ -1938,7 +1939,8 @@ __global__ void __launch_bounds__(NT) k_spectral(StepArgs a0) {
 // bin's annulus, taking kz and -kz together, so every mode is counted exactly
 // once and the sums are deterministic.  A bin narrower than a mode gives few
 // lanes one at a time: each warp lists its modes first and does the FP64 work
-// on full warps.  N=2048, 4096 bins: 1380 us with the formula per mode, 72 now.
+// on full warps.  N=2048, 4096 bins: 1380 us with the formula per mode, 73 now and
+// 6 for the edges.
 __device__ __forceinline__ int spectrum_bin(int k2, int nbins, double r_max, double k_nyq) {
   const double r = sqrt((double)k2) / k_nyq;
   const int bin = (int)floor((r / r_max) * (double)nbins);
